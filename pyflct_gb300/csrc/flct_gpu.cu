@@ -132,7 +132,7 @@ struct flct_ctx {
     }
     int bps[sizeof(kWin) / sizeof(kWin[0])][2] = {};
     int bps_tc[kNumTc][2] = {};
-    int bps_big = 0;
+    int bps_big[kMaxBigBox / 4 + 1] = {};  // by box side / 4
     Buf b_tc;              // tensor-core DFT matrices of every box size and split type
     size_t tc_off[kNumTc][2] = {};
     bool tc_ready = false;
@@ -349,6 +349,14 @@ int tc_bps(flct_ctx* ctx, int k, int which) {
     return ctx->bps_tc[k][which];
 }
 
+// CTAs per SM of the big-box kernel for box size n.
+int big_bps(flct_ctx* ctx, int n) {
+    if (n > kMaxBigBox) return 1;  // no kernel: launch_windows refuses it
+    int& b = ctx->bps_big[n / 4];
+    if (b == 0) b = std::max(1, window_big_blocks_per_sm(n));
+    return b;
+}
+
 // Resolve FLCT_FORM_AUTO (the autotuner's choice once it has measured box
 // size n, else the FP32 form) and check that the form exists for n.
 flct_status pick_form(flct_ctx* ctx, int requested, int n, int* form) {
@@ -408,8 +416,7 @@ flct_status launch_windows(flct_ctx* ctx, int form, const WinEntry* we, int n, c
                 ba.filt2[k] = (float)std::exp(-2.0 * ax * ax);
             }
         }
-        if (ctx->bps_big == 0) ctx->bps_big = std::max(1, window_big_blocks_per_sm(kMaxBigBox));
-        int grid = std::max(ctx->nsm, ctx->nsm * ctx->bps_big / grid_div);
+        int grid = std::max(ctx->nsm, ctx->nsm * big_bps(ctx, n) / grid_div);
         if (max_items >= 0) grid = (int)std::max<long>(1, max_items);
         CK(launch_window_big(ba, grid, st, pdl));
         return FLCT_OK;
@@ -923,7 +930,7 @@ flct_status enqueue_interp(flct_ctx* ctx, const Job& j, const JobBufs& b, cudaSt
 // a stream capture so the captured launches make none of these calls.
 flct_status prime_form(flct_ctx* ctx, int form, int n) {
     if (form == FLCT_FORM_FP32 && n > kMaxBox) {
-        if (ctx->bps_big == 0) ctx->bps_big = std::max(1, window_big_blocks_per_sm(kMaxBigBox));
+        big_bps(ctx, n);
         return FLCT_OK;
     }
     if (form == FLCT_FORM_FP32) {
