@@ -119,6 +119,15 @@ FLCT_HD float2 cfma(float2 a, float k, float2 b) {
         : "f"(a.x), "f"(a.y), "f"(k), "f"(b.x), "f"(b.y));
     return r;
 }
+// element-wise a * b + c
+FLCT_HD float2 efma(float2 a, float2 b, float2 c) {
+    float2 r;
+    asm("{\n.reg .b64 ra, rb, rc, rd;\nmov.b64 ra, {%2, %3};\nmov.b64 rb, {%4, %5};\nmov.b64 rc, {%6, %7};\n"
+        "fma.rn.f32x2 rd, ra, rb, rc;\nmov.b64 {%0, %1}, rd;\n}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
 #undef FLCT_PACKED_OP
 #else
 FLCT_HD float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
@@ -126,6 +135,7 @@ FLCT_HD float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.
 FLCT_HD float2 cfma(float2 a, float k, float2 b) { return make_float2(fmaf(a.x, k, b.x), fmaf(a.y, k, b.y)); }
 FLCT_HD float2 cscale(float2 a, float k) { return make_float2(a.x * k, a.y * k); }
 FLCT_HD float2 emul(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
+FLCT_HD float2 efma(float2 a, float2 b, float2 c) { return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)); }
 #endif
 // Scalar forms, for operands that are swapped or negated halves of a pair
 // (a packed instruction would first need them moved into a register pair).

@@ -966,27 +966,6 @@ void resolved_config(flct_ctx* ctx, int requested, int n, int* form, WinCfg* cfg
 
 // ------------------------------------------------------ sigma <= 0 --
 
-// make_freq (flct.c:1651-1690): 0..n/2-1, n/2 (and -n/2 for odd n), then
-// the negative frequencies.
-std::vector<double> make_freq(int n) {
-    std::vector<double> k(n);
-    const int n21 = n / 2 - 1;
-    int i = 0;
-    for (; i < n21 + 1; ++i) k[i] = (double)i;
-    int inext = n21 + 1;
-    if ((n / 2) * 2 != n) {
-        if (inext < n) k[inext] = (double)(n / 2);
-        ++inext;
-        if (inext < n) k[inext] = -(double)(n / 2);
-        ++inext;
-    } else {
-        if (inext < n) k[inext] = (double)(n / 2);
-        ++inext;
-    }
-    for (i = inext; i < n; ++i) k[i] = -(double)(n21 - (i - inext));
-    return k;
-}
-
 // The whole-frame correlation of the sigma <= 0 mode: FP64 means, FP32
 // batched DFTs, the same fits as the sliding windows (flct.c:802-942 with
 // init = 2).  Output: one (vx, vy, vm).
@@ -1002,33 +981,10 @@ flct_status velocity_global(flct_ctx* ctx, const Job& j, cudaStream_t st) {
     ENSURE(ctx->b_work, 64);
     ENSURE(ctx->b_peaks, sizeof(PeakRec));
     if (p->hires) ENSURE(ctx->b_peaks_h, sizeof(PeakRecH));
-    // twiddles e^{-2 pi i m / L} per axis and the squared -k filter factors
-    // exp(-2 (k / (kr k[L/2]))^2) (flct.c:1694-1715, applied to both spectra)
-    std::vector<unsigned char> tab((size_t)(nx + ny) * (sizeof(float2) + sizeof(float)));
-    float2* twx = (float2*)tab.data();
-    float2* twy = twx + nx;
-    float* fx2 = (float*)(twy + ny);
-    float* fy2 = fx2 + nx;
-    auto fill = [&](int L, float2* tw, float* f2) {
-        for (int m = 0; m < L; ++m) {
-            const double a = 2.0 * 3.14159265358979323846 * (double)m / (double)L;
-            tw[m] = make_float2((float)std::cos(a), (float)-std::sin(a));
-        }
-        const std::vector<double> k = make_freq(L);
-        const double roll = p->kr * k[L / 2];
-        for (int m = 0; m < L; ++m) {
-            const double ax = k[m] / roll;
-            f2[m] = p->filter ? (float)std::exp(-2.0 * ax * ax) : 1.0f;
-        }
-    };
-    fill(nx, twx, fx2);
-    fill(ny, twy, fy2);
-    unsigned char* dtab = (unsigned char*)ctx->b_b1.p;
-    CK(cudaMemcpyAsync(dtab, tab.data(), tab.size(), cudaMemcpyHostToDevice, st));
-    const float2* d_twx = (const float2*)dtab;
-    const float2* d_twy = d_twx + nx;
-    const float* d_fx2 = (const float*)(d_twy + ny);
-    const float* d_fy2 = d_fx2 + nx;
+    float2* d_twx = (float2*)ctx->b_b1.p;
+    float2* d_twy = d_twx + nx;
+    float* d_fx2 = (float*)(d_twy + ny);
+    float* d_fy2 = d_fx2 + nx;
     // counters: [0] nwork, [4] status, [8] peak key, [16] |g| maxima, [24] means
     unsigned char* ctr = (unsigned char*)ctx->b_ctr.p;
     int* d_nwork = (int*)ctr;
@@ -1042,36 +998,40 @@ flct_status velocity_global(flct_ctx* ctx, const Job& j, cudaStream_t st) {
     ctx->batch_pending = 0;
     CK(cudaEventRecord(ctx->ev[0], st));
     CK(cudaMemsetAsync(ctr, 0, 64, st));
-    k_gsum_part<<<kGsumBlocks, 256, 0, st>>>(j.f1, j.f2, n, (double*)ctx->b_aux2.p);
-    k_gsum_final<<<1, 256, 0, st>>>((const double*)ctx->b_aux2.p, kGsumBlocks, (double)nx * ny, d_means);
+    // every kernel as a programmatic dependent of the one before (each waits
+    // for it before its first global access): the chain is short kernels
+    CK(launch_kernel(k_gtables, dim3((nx + ny + 127) / 128), dim3(128), 0, st, true, nx, ny, p->filter, p->kr, d_twx,
+                     d_twy, d_fx2, d_fy2));
+    CK(launch_kernel(k_gsum_part, dim3(kGsumBlocks), dim3(256), 0, st, true, j.f1, j.f2, n, (double*)ctx->b_aux2.p));
+    CK(launch_kernel(k_gsum_final, dim3(1), dim3(256), 0, st, true, (const double*)ctx->b_aux2.p, kGsumBlocks,
+                     (double)nx * ny, d_means));
     const int eblocks = (int)std::min<long>((n + 255) / 256, (long)ctx->nsm * 8);
-    k_gz<<<eblocks, 256, 0, st>>>(j.f1, j.f2, n, d_means, A, d_max, d_status);
-    launches += 3;
-    CK(cudaGetLastError());
+    CK(launch_kernel(k_gz, dim3(eblocks), dim3(256), 0, st, true, j.f1, j.f2, n, d_means, A, d_max, d_status));
+    launches += 4;
     CK(cudaEventRecord(ctx->ev[1], st));
-    auto dft = [&](bool inverse, const float2* in, float2* out, int L, int lines, const float2* tw,
-                   const unsigned* sc) {
-        launch_dft_rows(inverse, in, out, L, lines, tw, sc, st);
+    auto dft = [&](bool inverse, bool real_out, const float2* in, float2* out, int axis, const unsigned* sc) {
         ++launches;
+        return launch_dft_rows(inverse, real_out, in, out, axis ? ny : nx, axis ? nx : ny, axis ? d_twy : d_twx, sc,
+                               ctx->nsm, st);
     };
     auto transpose = [&](const float2* in, float2* out, int R, int C) {
-        k_transpose<<<dim3((C + 31) / 32, (R + 31) / 32), dim3(32, 8), 0, st>>>(in, out, R, C);
         ++launches;
+        return launch_kernel(k_transpose, dim3((C + 31) / 32, (R + 31) / 32), dim3(32, 8), 0, st, true, in, out, R, C);
     };
-    dft(false, A, B, ny, nx, d_twy, d_max);  // along the fast axis, with the power-of-two scales
-    transpose(B, A, nx, ny);                 // [ky][i]
-    dft(false, A, B, nx, ny, d_twx, nullptr);  // Zt[ky][kx]
-    k_gprod<<<eblocks, 256, 0, st>>>(B, A, nx, ny, d_fx2, d_fy2);
+    CK(dft(false, false, A, B, 1, d_max));    // along the fast axis, with the power-of-two scales
+    CK(transpose(B, A, nx, ny));              // [ky][i]
+    CK(dft(false, false, A, B, 0, nullptr));  // Zt[ky][kx]
+    CK(launch_kernel(k_gprod, dim3(eblocks), dim3(256), 0, st, true, B, A, nx, ny, d_fx2, d_fy2));
     ++launches;
-    dft(true, A, B, nx, ny, d_twx, nullptr);
-    transpose(B, A, ny, nx);
-    dft(true, A, B, ny, nx, d_twy, nullptr);  // c[i][j] (real part)
-    k_gpeak<<<eblocks, 256, 0, st>>>(B, nx, ny, d_key);
+    CK(dft(true, false, A, B, 0, nullptr));
+    CK(transpose(B, A, ny, nx));
+    CK(dft(true, true, A, B, 1, nullptr));  // c[i][j], the real part
+    CK(launch_kernel(k_gpeak, dim3(eblocks), dim3(256), 0, st, true, B, nx, ny, d_key));
     PeakRec* rec = (PeakRec*)ctx->b_peaks.p;
     PeakRecH* rech = p->hires ? (PeakRecH*)ctx->b_peaks_h.p : nullptr;
-    k_gpatch<<<1, 64, 0, st>>>(B, nx, ny, d_key, rec, rech, (int*)ctx->b_work.p, d_nwork);
+    CK(launch_kernel(k_gpatch, dim3(1), dim3(64), 0, st, true, B, nx, ny, d_key, rec, rech, (int*)ctx->b_work.p,
+                     d_nwork));
     launches += 2;
-    CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev[2], st));
     FitArgs fa{};
     fa.work = (const int*)ctx->b_work.p;
@@ -1086,10 +1046,9 @@ flct_status velocity_global(flct_ctx* ctx, const Job& j, cudaStream_t st) {
     fa.vx = j.vx;
     fa.vy = j.vy;
     fa.vm = j.vm;
-    if (rech) k_fit_hires<<<1, 128, 0, st>>>(fa);
-    else k_fit<<<1, 32, 0, st>>>(fa);
+    if (rech) CK(launch_kernel(k_fit_hires, dim3(1), dim3(128), 0, st, true, fa));
+    else CK(launch_kernel(k_fit, dim3(1), dim3(32), 0, st, true, fa));
     ++launches;
-    CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev[7], st));
     CK(cudaMemcpyAsync(ctx->hctr, ctr, 8, cudaMemcpyDeviceToHost, st));
     CK(cudaEventRecord(ctx->ev[3], st));

@@ -1,6 +1,9 @@
 // global.cu -- kernels of the sigma <= 0 mode (see global.cuh).
 #include "global.cuh"
 
+#include "fft_reg.cuh"
+#include "warp_math.cuh"
+
 namespace flct {
 
 __device__ __forceinline__ double warp_sum_d(double v) {
@@ -30,6 +33,7 @@ __device__ __forceinline__ void block_sum2(double& a, double& b) {
 
 __global__ void k_gsum_part(const double* __restrict__ f1, const double* __restrict__ f2, long n,
                             double* __restrict__ part) {
+    grid_dep_wait();
     const long chunk = (n + gridDim.x - 1) / gridDim.x;
     const long b0 = blockIdx.x * chunk, b1 = min(n, b0 + chunk);
     double a = 0., b = 0.;
@@ -45,6 +49,7 @@ __global__ void k_gsum_part(const double* __restrict__ f1, const double* __restr
 }
 
 __global__ void k_gsum_final(const double* __restrict__ part, int nparts, double dn, double* __restrict__ means) {
+    grid_dep_wait();
     double a = 0., b = 0.;
     for (int k = threadIdx.x; k < nparts; k += blockDim.x) {
         a = __dadd_rn(a, part[2 * k]);
@@ -60,6 +65,7 @@ __global__ void k_gsum_final(const double* __restrict__ part, int nparts, double
 __global__ void k_gz(const double* __restrict__ f1, const double* __restrict__ f2, long n,
                      const double* __restrict__ means, float2* __restrict__ z, unsigned* maxbits,
                      unsigned* status) {
+    grid_dep_wait();
     const float2 m1 = split_double_fast(means[0]), m2 = split_double_fast(means[1]);
     float mx1 = 0.f, mx2 = 0.f;
     for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
@@ -84,52 +90,139 @@ __global__ void k_gz(const double* __restrict__ f1, const double* __restrict__ f
     }
 }
 
-constexpr int kDftChunk = 2048;
+// Tile of a direct DFT: 32 LP lines by 16 KQ frequencies, LP pairs of lines
+// by KQ frequencies per thread, on packed FMAs (two lines an instruction).
+// Every output adds its L terms from j = 0 up, the real part x.x w.x after
+// -x.y w.y, so results do not depend on the tile.  Chunks of kDftChunk points
+// of the lines and their twiddles tw[(j k) mod L] go through shared memory;
+// a thread steps the index of its twiddle column.  Bound by the FP32 pipe (65% busy; 4 FMAs per point and output, 2
+// where only the real part is wanted).  The four passes of a 1000 x 1200
+// call: 5.1 -> 0.83 ms against one output a thread, which read the table once
+// per 4 FMAs.
+constexpr int kDftChunk = 16;
 
-template <int DIR>
+template <int DIR, int LP, int KQ, bool REAL_OUT>
 __global__ void __launch_bounds__(256) k_dft_rows(const float2* __restrict__ in, float2* __restrict__ out, int L,
                                                   int lines, const float2* __restrict__ tw,
                                                   const unsigned* __restrict__ scale) {
-    __shared__ float2 s_x[kDftChunk];
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = k < L;
+    constexpr int J = kDftChunk, WL = 32 * LP, WK = 16 * KQ;
+    __shared__ __align__(16) float xr[J][WL + 2], xi[J][WL + 2];
+    __shared__ float2 ws[J][WK];
+    grid_dep_wait();
+    // a thread's outputs lie 16 frequencies (32 lines) apart, so that a warp
+    // reads whole rows of ws
+    const int t = threadIdx.x, tk = t & 15, tl = 2 * (t >> 4);
+    const int k0 = blockIdx.x * WK, l0 = blockIdx.y * WL;
     const float c1 = scale ? pow2_scale(scale[0]) : 1.f, c2 = scale ? pow2_scale(scale[1]) : 1.f;
-    for (int line = blockIdx.y; line < lines; line += gridDim.y) {
-        const float2* src = in + (size_t)line * L;
-        float ax = 0.f, ay = 0.f;
-        for (int j0 = 0; j0 < L; j0 += kDftChunk) {
-            const int cnt = min(kDftChunk, L - j0);
-            __syncthreads();
-            for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
-                const float2 v = src[j0 + t];
-                s_x[t] = make_float2(v.x * c1, v.y * c2);
-            }
-            __syncthreads();
-            if (active) {
-                int idx = (int)(((long)j0 * k) % L);  // (j k) mod L, stepped by k
-                for (int t = 0; t < cnt; ++t) {
-                    float2 w = __ldg(tw + idx);
-                    if (DIR > 0) w.y = -w.y;
-                    const float2 x = s_x[t];
-                    ax = fmaf(x.x, w.x, fmaf(-x.y, w.y, ax));
-                    ay = fmaf(x.x, w.y, fmaf(x.y, w.x, ay));
-                    idx += k;
-                    if (idx >= L) idx -= L;
-                }
-            }
+    // this thread's twiddle column, from its row on
+    constexpr int WR = 256 / WK;  // twiddle rows a round
+    const int wk = t % WK, wj = t / WK, k = min(k0 + wk, L - 1);
+    int idx = (int)((long)wj * k % L);
+    const int step = (int)((long)WR * k % L);
+    float2 ax[LP][KQ] = {}, ay[LP][KQ] = {};
+    // the next chunk travels while this one is summed; half a warp reads 16
+    // points of a line
+    constexpr int NX = WL * J / 256, NW = J / WR;
+    const int jx = t % J, lx = t / J;
+    float2 nx[NX], nw[NW];
+    auto fetch = [&](int j0) {
+#pragma unroll
+        for (int q = 0; q < NX; ++q) {
+            const int l = l0 + lx + q * (256 / J);
+            nx[q] = (l < lines && j0 + jx < L) ? __ldg(in + (size_t)l * L + j0 + jx) : make_float2(0.f, 0.f);
         }
-        if (active) out[(size_t)line * L + k] = make_float2(ax, ay);
+#pragma unroll
+        for (int q = 0; q < NW; ++q) {
+            nw[q] = __ldg(tw + idx);
+            idx += step;
+            if (idx >= L) idx -= L;
+        }
+    };
+    fetch(0);
+    for (int j0 = 0; j0 < L; j0 += J) {
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < NX; ++q) {
+            xr[jx][lx + q * (256 / J)] = nx[q].x * c1;
+            xi[jx][lx + q * (256 / J)] = nx[q].y * c2;
+        }
+#pragma unroll
+        for (int q = 0; q < NW; ++q) {
+            ws[wj + q * WR][wk] = make_float2(nw[q].x, DIR > 0 ? -nw[q].y : nw[q].y);
+        }
+        __syncthreads();
+        if (j0 + J < L) fetch(j0 + J);
+        const int jn = min(J, L - j0);
+#pragma unroll 4
+        for (int j = 0; j < jn; ++j) {
+            float2 re[LP], im[LP], ni[LP];
+            float2 w[KQ];
+#pragma unroll
+            for (int p = 0; p < LP; ++p) {
+                re[p] = *reinterpret_cast<const float2*>(&xr[j][tl + 32 * p]);
+                im[p] = *reinterpret_cast<const float2*>(&xi[j][tl + 32 * p]);
+                ni[p] = make_float2(-im[p].x, -im[p].y);
+            }
+#pragma unroll
+            for (int q = 0; q < KQ; ++q) w[q] = ws[j][tk + 16 * q];
+#pragma unroll
+            for (int p = 0; p < LP; ++p)
+#pragma unroll
+                for (int q = 0; q < KQ; ++q) {
+                    const float2 wx = make_float2(w[q].x, w[q].x), wy = make_float2(w[q].y, w[q].y);
+                    ax[p][q] = efma(re[p], wx, efma(ni[p], wy, ax[p][q]));
+                    if (!REAL_OUT) ay[p][q] = efma(re[p], wy, efma(im[p], wx, ay[p][q]));
+                }
+        }
     }
+#pragma unroll
+    for (int p = 0; p < LP; ++p)
+#pragma unroll
+        for (int q = 0; q < KQ; ++q) {
+            const int l = l0 + tl + 32 * p, kk = k0 + tk + 16 * q;
+            if (kk >= L) continue;
+            if (l < lines) out[(size_t)l * L + kk] = make_float2(ax[p][q].x, ay[p][q].x);
+            if (l + 1 < lines) out[(size_t)(l + 1) * L + kk] = make_float2(ax[p][q].y, ay[p][q].y);
+        }
 }
-cudaError_t launch_dft_rows(bool inverse, const float2* in, float2* out, int L, int lines, const float2* tw,
-                            const unsigned* scale, cudaStream_t st) {
-    const dim3 g((L + 255) / 256, lines < 65535 ? lines : 65535);
-    if (inverse) k_dft_rows<1><<<g, 256, 0, st>>>(in, out, L, lines, tw, scale);
-    else k_dft_rows<-1><<<g, 256, 0, st>>>(in, out, L, lines, tw, scale);
-    return cudaGetLastError();
+
+cudaError_t launch_dft_rows(bool inverse, bool real_out, const float2* in, float2* out, int L, int lines,
+                            const float2* tw, const unsigned* scale, int nsm, cudaStream_t st) {
+    // the widest tile that still gives every SM one
+    auto grid = [&](int wl, int wk) { return dim3((L + wk - 1) / wk, (lines + wl - 1) / wl); };
+    auto tiles = [&](int wl, int wk) { return (long)grid(wl, wk).x * grid(wl, wk).y; };
+    const bool wide = tiles(64, 64) >= nsm, mid = tiles(32, 32) >= nsm;
+#define FLCT_DFT(D, LP, KQ, R) \
+    launch_kernel(k_dft_rows<D, LP, KQ, R>, grid(32 * LP, 16 * KQ), dim3(256), 0, st, true, in, out, L, lines, tw, scale)
+#define FLCT_DFT_TILE(D, R) (wide ? FLCT_DFT(D, 2, 4, R) : mid ? FLCT_DFT(D, 1, 2, R) : FLCT_DFT(D, 1, 1, R))
+    return !inverse ? FLCT_DFT_TILE(-1, false) : real_out ? FLCT_DFT_TILE(1, true) : FLCT_DFT_TILE(1, false);
+#undef FLCT_DFT_TILE
+#undef FLCT_DFT
+}
+
+// Twiddles e^{-2 pi i m / L} of both axes and the squared -k filter factors
+// exp(-2 (k / (kr n / 2))^2) by frequency index (flct.c:1694-1715, applied to
+// both spectra; 1 without -k).
+__global__ void k_gtables(int nx, int ny, int use, double kr, float2* __restrict__ twx, float2* __restrict__ twy,
+                          float* __restrict__ fx2, float* __restrict__ fy2) {
+    grid_dep_wait();
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= nx + ny) return;
+    const int n = e < nx ? nx : ny, k = e < nx ? e : e - nx;
+    const double a = 2.0 * 3.14159265358979323846 * (double)k / (double)n;
+    double s, c;
+    sincos(a, &s, &c);
+    (e < nx ? twx : twy)[k] = make_float2((float)c, (float)-s);
+    float f = 1.0f;
+    if (use) {
+        const double x = (double)freq_of(k, n) / (kr * (double)(n / 2));
+        f = (float)exp(-2.0 * x * x);
+    }
+    (e < nx ? fx2 : fy2)[k] = f;
 }
 
 __global__ void k_transpose(const float2* __restrict__ in, float2* __restrict__ out, int R, int C) {
+    grid_dep_wait();
     __shared__ float2 t[32][33];
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
     for (int dy = threadIdx.y; dy < 32; dy += blockDim.y) {
@@ -145,6 +238,7 @@ __global__ void k_transpose(const float2* __restrict__ in, float2* __restrict__ 
 
 __global__ void k_gprod(const float2* __restrict__ zt, float2* __restrict__ ct, int nx, int ny,
                         const float* __restrict__ fx2, const float* __restrict__ fy2) {
+    grid_dep_wait();
     const long n = (long)nx * ny;
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
         const int ky = (int)(e / nx), kx = (int)(e - (long)ky * nx);
@@ -158,6 +252,7 @@ __global__ void k_gprod(const float2* __restrict__ zt, float2* __restrict__ ct, 
 }
 
 __global__ void k_gpeak(const float2* __restrict__ c, int nx, int ny, unsigned long long* key) {
+    grid_dep_wait();
     const long n = (long)nx * ny;
     unsigned long long best = 0ull;
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
@@ -179,6 +274,7 @@ __global__ void k_gpeak(const float2* __restrict__ c, int nx, int ny, unsigned l
 
 __global__ void k_gpatch(const float2* __restrict__ c, int nx, int ny, const unsigned long long* __restrict__ key,
                          PeakRec* rec, PeakRecH* rech, int* work, int* nwork) {
+    grid_dep_wait();
     // |c| at shifted coordinates (I, J)
     auto sh = [&](int I, int J) -> float {
         const int i = (I - nx / 2 + nx) % nx, j = (J - ny / 2 + ny) % ny;

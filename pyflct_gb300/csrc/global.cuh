@@ -2,12 +2,12 @@
 // whole frames (flct.c:581-586, 666-675, 802-808).
 //
 // The frames are mean-subtracted (FP64 means), packed as z = g1 + i g2 in
-// FP32 (hi + lo split, scaled by a power of two), transformed by batched
-// direct DFTs along each axis (any size; exact twiddle tables built on the
-// host), separated into conj(A) B with the mirror trick and the -k filter,
-// transformed back, and |c| searched for its first strict maximum in the
-// half-shifted frame.  The peak record then goes through the same k_fit /
-// k_fit_hires as the sliding windows.
+// FP32 (hi + lo split, scaled by a power of two), transformed by tiled direct
+// DFTs along each axis (any size; exact twiddle tables), separated into
+// conj(A) B with the mirror trick and the -k filter, transformed back, and
+// |c| searched for its first strict maximum in the half-shifted frame.  The
+// peak record then goes through the same k_fit / k_fit_hires as the sliding
+// windows.
 #pragma once
 #include "common.cuh"
 #include "window_common.cuh"
@@ -27,9 +27,12 @@ __global__ void k_gz(const double* f1, const double* f2, long n, const double* m
 
 // out[l][k] = sum_j in[l][j] tw[(j k) mod L]^dir, lines of length L
 // contiguous (stride L); with `scale` the inputs are first multiplied by
-// (pow2_scale(scale[0]), pow2_scale(scale[1])) per component.
-cudaError_t launch_dft_rows(bool inverse, const float2* in, float2* out, int L, int lines, const float2* tw,
-                            const unsigned* scale, cudaStream_t st);
+// (pow2_scale(scale[0]), pow2_scale(scale[1])) per component.  real_out: only
+// the real part is wanted (the imaginary part is written as 0).
+cudaError_t launch_dft_rows(bool inverse, bool real_out, const float2* in, float2* out, int L, int lines,
+                            const float2* tw, const unsigned* scale, int nsm, cudaStream_t st);
+
+__global__ void k_gtables(int nx, int ny, int use, double kr, float2* twx, float2* twy, float* fx2, float* fy2);
 
 // out[c][r] = in[r][c] for an R x C array.
 __global__ void k_transpose(const float2* in, float2* out, int R, int C);
