@@ -966,6 +966,22 @@ void resolved_config(flct_ctx* ctx, int requested, int n, int* form, WinCfg* cfg
 
 // ------------------------------------------------------ sigma <= 0 --
 
+size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+// Both axes' line plans (0 slow, 1 fast) and the bytes of their tables.
+// Lengths with a prime factor above 13 take a chirp from chirp_min points on.
+LineSetup line_setup(int nx, int ny, int chirp_min) {
+    LineSetup s;
+    s.p[0] = line_plan(nx, chirp_min);
+    s.p[1] = line_plan(ny, chirp_min);
+    return s;
+}
+size_t line_setup_bytes(const LineSetup& s) { return align256(line_tab_bytes(s.p[0])) + line_tab_bytes(s.p[1]); }
+void place_tables(LineSetup* s, void* mem) {
+    s->t[0] = line_tab(s->p[0], mem);
+    s->t[1] = line_tab(s->p[1], static_cast<unsigned char*>(mem) + align256(line_tab_bytes(s->p[0])));
+}
+
 // The whole-frame correlation of the sigma <= 0 mode: FP64 means, FP32
 // batched DFTs, the same fits as the sliding windows (flct.c:802-942 with
 // init = 2).  Output: one (vx, vy, vm).
@@ -1095,8 +1111,6 @@ struct BatchPlan {
     int* first = nullptr;    // device, ngroups + 1
     std::vector<int> h_first;
 };
-
-size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // The fields of a pair list that a captured batch depends on.
 std::vector<unsigned char> batch_key(int npairs, const flct_pair* pairs) {
@@ -2468,20 +2482,28 @@ flct_status flct_gpu_shift_frac2d(flct_ctx* ctx, const double* arr, double delx,
     ENSURE(ctx->b_vx, n * sizeof(double));
     ENSURE(ctx->b_s1, n * sizeof(float2));
     ENSURE(ctx->b_s2, n * sizeof(float2));
-    ENSURE(ctx->b_aux1, (size_t)(nx + ny) * sizeof(float2) + 64);
+    // the circulant vectors are quicker on short rough axes (37 x 53: 50
+    // against 58 us of kernels; 97 x 101: 78 against 60)
+    LineSetup ls = line_setup(nx, ny, 64);
+    const bool fft = ls.p[0].npass && ls.p[1].npass;
+    ENSURE(ctx->b_aux1, fft ? line_setup_bytes(ls) : (size_t)(nx + ny) * sizeof(float2) + 64);
     ENSURE(ctx->b_aux2, (size_t)2 * (nx + ny) * sizeof(double2));
     float2* sx = (float2*)ctx->b_aux1.p;
     float2* sy = sx + nx;
     // warp.c:811-820: shifts normalised by the axis lengths; transp swaps them
     const double dxarg = transp ? -dely / ((double)nx) : -delx / ((double)nx);
     const double dyarg = transp ? -delx / ((double)ny) : -dely / ((double)ny);
-    const bool fft = shift_fft_axis(nx) && shift_fft_axis(ny);
     CK(cudaMemcpyAsync(ctx->b_f1.p, arr, n * sizeof(double), cudaMemcpyHostToDevice, st));
     CK(cudaEventRecord(ctx->ev[0], st));
     if (fft) {
-        // power-of-two axes: the same linear map by transforms, O(N log N)
-        CK(launch_shift_fft((const double*)ctx->b_f1.p, nx, ny, dxarg, dyarg, (double2*)ctx->b_aux2.p, sx,
-                            (float2*)ctx->b_s1.p, (float2*)ctx->b_s2.p, (double*)ctx->b_vx.p, ctx->nsm, st));
+        // the same linear map by transforms, O(N log N)
+        place_tables(&ls, ctx->b_aux1.p);
+        ls.darg[0] = dxarg;
+        ls.darg[1] = dyarg;
+        ls.ph[0] = (double2*)ctx->b_aux2.p;
+        ls.ph[1] = ls.ph[0] + nx;
+        CK(launch_shift_fft((const double*)ctx->b_f1.p, ls, (float2*)ctx->b_s1.p, (float2*)ctx->b_s2.p,
+                            (double*)ctx->b_vx.p, ctx->nsm, st));
     } else {
         CK(launch_shift_vector(nx, dxarg, (double2*)ctx->b_aux2.p, sx, st));
         CK(launch_shift_vector(ny, dyarg, (double2*)ctx->b_aux2.p, sy, st));
@@ -2493,7 +2515,7 @@ flct_status flct_gpu_shift_frac2d(flct_ctx* ctx, const double* arr, double delx,
     CK(cudaMemcpyAsync(out, ctx->b_vx.p, n * sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     ctx->timing = flct_timing{};
-    ctx->timing.launches = fft ? 8 : 7;
+    ctx->timing.launches = fft ? 5 + (ls.p[0].chirp || ls.p[1].chirp) : 7;
     ctx->timing.ms_total = ev_ms(ctx->ev[0], ctx->ev[1]);
     return FLCT_OK;
 }
@@ -2514,19 +2536,20 @@ flct_status flct_gpu_warp_frac2d(flct_ctx* ctx, const double* arr, const double*
     ENSURE(ctx->b_s1, n * sizeof(float2));
     ENSURE(ctx->b_s2, n * sizeof(float2));
     ENSURE(ctx->b_means, n * sizeof(float4));
-    ENSURE(ctx->b_aux1, (size_t)(nx + ny) * sizeof(float2) + 64);
+    LineSetup ls = line_setup(nx, ny, 1);
+    const bool fft = ls.p[0].npass && ls.p[1].npass;
+    ENSURE(ctx->b_aux1, fft ? line_setup_bytes(ls) : (size_t)(nx + ny) * sizeof(float2) + 64);
     float2* twx = (float2*)ctx->b_aux1.p;
     float2* twy = twx + nx;
     CK(cudaMemcpyAsync(ctx->b_f1.p, arr, n * sizeof(double), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(ctx->b_f2.p, delx, n * sizeof(double), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(ctx->b_vy.p, dely, n * sizeof(double), cudaMemcpyHostToDevice, st));
     CK(cudaEventRecord(ctx->ev[0], st));
-    // F = forward DFT of the image (warp.c:899-934): FFTs along both axes
-    // when both are powers of two (64 .. kWarpMaxAxis), else DFT matrices
-    const bool fft = shift_fft_axis(nx) && shift_fft_axis(ny);
+    // F = forward DFT of the image (warp.c:899-934): transforms along both
+    // axes where both have line plans, else DFT matrices
     if (fft) {
-        CK(launch_dft2_fft((const double*)ctx->b_f1.p, nx, ny, twx, (float2*)ctx->b_s1.p, (float2*)ctx->b_s2.p,
-                           ctx->nsm, st));
+        place_tables(&ls, ctx->b_aux1.p);
+        CK(launch_dft2_fft((const double*)ctx->b_f1.p, ls, (float2*)ctx->b_s1.p, (float2*)ctx->b_s2.p, ctx->nsm, st));
     } else {
         CK(launch_twiddles(nx, -1, twx, st));
         CK(launch_twiddles(ny, -1, twy, st));
@@ -2557,7 +2580,7 @@ flct_status flct_gpu_warp_frac2d(flct_ctx* ctx, const double* arr, const double*
     if (tc) CK(cudaMemcpyAsync(&wstatus, (unsigned*)ctx->b_wmisc.p + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     ctx->timing = flct_timing{};
-    ctx->timing.launches = (fft ? 6 : 4) + 1 + (tc ? 3 : 1);
+    ctx->timing.launches = (fft ? 5 + (ls.p[0].chirp || ls.p[1].chirp) : 4) + 1 + (tc ? 3 : 1);
     ctx->timing.ms_prepass = ev_ms(ctx->ev[0], ctx->ev[1]);
     ctx->timing.ms_window = ev_ms(ctx->ev[1], ctx->ev[2]);
     ctx->timing.ms_total = ev_ms(ctx->ev[0], ctx->ev[2]);
