@@ -834,11 +834,12 @@ void make_wargs(const Job& j, const JobBufs& b, WinArgs* wa) {
     wa->use_filter = j.p->filter;
     wa->s12 = b.s12;
     wa->means = b.means;
-    wa->mg = MeanGrid{j.gs, j.xo, j.yo, j.gj};
+    wa->mg = MeanGrid{FastDiv(j.gs), j.xo, j.yo, j.gj};
     wa->work = b.work;
     wa->nwork = (const int*)b.ctr;
     wa->nx = j.nx;
     wa->ny = j.ny;
+    wa->nyd = FastDiv(j.ny);
     wa->nsize = j.d.nsize;
     wa->peaks = b.peaks;
     wa->peaks_h = j.p->hires ? b.peaks_h : nullptr;
@@ -1343,9 +1344,9 @@ flct_status plan_batch(flct_ctx* ctx, int npairs, const flct_pair* pairs, BatchP
             WinSeg sg{};
             sg.s12 = bp->bufs[k].s12;
             sg.nx = bp->jobs[k].nx;
-            sg.ny = bp->jobs[k].ny;
+            sg.ny = FastDiv(bp->jobs[k].ny);
             sg.base = (int)off[k].base;
-            sg.mg = MeanGrid{bp->jobs[k].gs, bp->jobs[k].xo, bp->jobs[k].yo, bp->jobs[k].gj};
+            sg.mg = MeanGrid{FastDiv(bp->jobs[k].gs), bp->jobs[k].xo, bp->jobs[k].yo, bp->jobs[k].gj};
             hs[e] = sg;
             hpair[e] = k;
             ++e;
@@ -2377,6 +2378,7 @@ flct_status flct_gpu_cross_cor_batch(flct_ctx* ctx, const double* g1, const doub
     wa.nwork = (const int*)ctr;
     wa.nx = nwin * n;
     wa.ny = n;
+    wa.nyd = FastDiv(n);
     wa.nsize = n / 2;
     wa.direct = 1;
     ENSURE(ctx->b_peaks, (size_t)nwin * sizeof(PeakRec));

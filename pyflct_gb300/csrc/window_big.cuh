@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(BigShape<M>::THREADS, BigShape<M>::MINB) k_win
             const WinSeg sg = a.segs[k];
             f12 = sg.s12;
             nx = sg.nx;
-            ny = sg.ny;
+            ny = sg.ny.d;
             if (mp) mp += sg.base;
             mg = sg.mg;
             gi = sg.base + (gi - __ldg(a.seg_start + k));

@@ -42,6 +42,7 @@ struct WinArgs {
     const int* work;      // pixel indices i*ny + j
     const int* nwork;     // number of work items (device)
     int nx, ny, nsize;
+    FastDiv nyd;          // ny again
     int use_filter;       // -k given
     int direct;           // windows given directly: box w starts at row w*n, unit weights
     PeakRec* peaks;       // per work item: integer peak and its 3x3 |c| stencil
@@ -61,10 +62,28 @@ struct WinArgs {
 // else half the teams, with no register cap.  A window's arithmetic is the
 // same in both; only the windows per CTA and the occupancy differ.
 template <int N>
-constexpr int win_teams0() { return (N <= 8) ? (128 / N) : (N <= 20 || N == 32) ? 8 : (N <= 40) ? 4 : 2; }
+constexpr int win_teams0() {
+    return (N <= 8) ? (128 / N) : (N <= 20 || N == 32) ? 8 : (N <= 44) ? 4 : 2;
+}
+// Boxes 16 and 32 (whole-warp teams) read rows and row weights 16 bytes at a
+// time and look for the peak's place only after its value: 8% fewer
+// instructions at box 32, which also brings its loop inside the instruction
+// cache (29 KB of code; at 32 KB it asked the cache behind for 57% of its
+// bandwidth).  65,536 windows: box 16 44.7 -> 42.7 us, box 32 165.6 -> 159.4.
+// Boxes 4 and 8 gain nothing by it (9.9 -> 11.9, 17.7 -> 18.0), and teams that
+// share warps pay more for the peak's second look than they save.
+template <int N>
+constexpr bool win_quads() { return N == 16 || N == 32; }
+// 16-byte row reads want a stride of n + 2 to stay on distinct banks, 8-byte
+// ones n + 1; the row weights are four shifted copies, read from any start.
+template <int N>
+constexpr int win_ld() { return win_quads<N>() ? N + 2 : N + 1; }
+template <int N>
+constexpr size_t win_weights() { return win_quads<N>() ? (size_t)4 * (N / 2 + 1) * 16 : 0; }
 template <int N>
 constexpr size_t win_smem(int teams) {
-    return 32 * teams + ((3 * N + 1) * 4 + 15) / 16 * 16 + (size_t)N * 8 + (size_t)teams * N * (N + 1) * 8;
+    return 32 * teams + win_weights<N>() + ((3 * N + 1) * 4 + 15) / 16 * 16 + (size_t)N * 8 +
+           (size_t)teams * N * win_ld<N>() * 8;
 }
 template <int N>
 constexpr int win_teams_alt() {
@@ -76,28 +95,37 @@ template <int N, int V = 0>
 struct WinShape {
     static constexpr int TEAMS = V == 0 ? win_teams0<N>() : win_teams_alt<N>();
     static constexpr int THREADS = N * TEAMS;
-    static constexpr int BUF = N * (N + 1);  // float2 per team
-    static constexpr size_t tw_off = 32 * TEAMS + ((3 * N + 1) * 4 + 15) / 16 * 16;
+    static constexpr int LD = win_ld<N>();   // row stride, float2
+    static constexpr int BUF = N * LD;       // float2 per team
+    static constexpr size_t g_off = 32 * TEAMS + win_weights<N>();
+    static constexpr size_t tw_off = g_off + ((3 * N + 1) * 4 + 15) / 16 * 16;
     static constexpr size_t head = tw_off + (size_t)N * 8;
     static constexpr size_t smem = head + (size_t)TEAMS * BUF * 8;  // |c| reuses the buffer
     static_assert(smem == win_smem<N>(TEAMS), "shared-memory layout");
     // CTAs per SM the register allocation is held to (0: no constraint).
-    // Box 32: 2 CTAs of 8 teams at 128 registers, no spills, beat 5 CTAs of
-    // 4 teams at 96 registers with 12 bytes spilled (175.8 against 181.9 us
-    // for 65,536 windows; 4 CTAs of 4 teams at 128 registers: 179.9 us;
-    // measured).
-    static constexpr int MINB = (V == 0 && N == 32) ? 2 : 0;
+    // Box 32: 2 CTAs of 8 teams at 128 registers (159.5 us for 65,536 windows;
+    // 161.4 at 20 warps per SM, 190 at 12).  Box 16: 7 CTAs of 4 warps (46.8
+    // us at 16 warps per SM, 42.6 at 28).
+    static constexpr int MINB = V == 0 ? (N == 32 ? 2 : N == 16 ? 7 : 0) : 0;
 };
+
+// max(|a|, |b|, |c|), NaN ignored (one instruction)
+__device__ __forceinline__ float max3_abs(float a, float b, float c) {
+    float r;
+    asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
 
 template <int N, int V>
 __global__ void __launch_bounds__(WinShape<N, V>::THREADS, WinShape<N, V>::MINB)
 k_window_fp32(WinArgs a) {
     using S = WinShape<N, V>;
-    constexpr int TEAMS = S::TEAMS;
+    constexpr int TEAMS = S::TEAMS, LD = S::LD;
     extern __shared__ __align__(16) unsigned char sm[];
     unsigned long long* s_key = reinterpret_cast<unsigned long long*>(sm + 16 * TEAMS);
     unsigned* s_max = reinterpret_cast<unsigned*>(sm + 24 * TEAMS);
-    float* s_g = reinterpret_cast<float*>(sm + 32 * TEAMS);
+    float4* s_g4 = reinterpret_cast<float4*>(sm + 32 * TEAMS);  // copy c, entry m: row weights 4 m + c ..
+    float* s_g = reinterpret_cast<float*>(sm + S::g_off);
     float* s_f = s_g + (2 * N + 1);
     float2* s_tw = reinterpret_cast<float2*>(sm + S::tw_off);  // e^{2 pi i k / N}
     float2* s_buf = reinterpret_cast<float2*>(sm + S::head);
@@ -109,6 +137,7 @@ k_window_fp32(WinArgs a) {
     // shuffles; other team widths share warps and go through shared memory
     // and the CTA barrier.
     constexpr bool kWarp = (32 % N == 0);
+    constexpr bool kQuads = win_quads<N>();
     const unsigned tmask =
         (N == 32) ? 0xffffffffu : (((1u << (N & 31)) - 1u) << ((threadIdx.x & 31) & ~(unsigned)(N - 1)));
     auto team_sync = [] {
@@ -116,6 +145,13 @@ k_window_fp32(WinArgs a) {
         else __syncthreads();
     };
     for (int k = threadIdx.x; k < 2 * N + 1; k += blockDim.x) s_g[k] = a.gauss[k];
+    if constexpr (kQuads) {
+        for (int k = threadIdx.x; k < 4 * (N / 2 + 1); k += blockDim.x) {
+            const int r = 4 * (k % (N / 2 + 1)) + k / (N / 2 + 1);
+            auto g = [&](int q) { return q <= 2 * N ? a.gauss[q] : 0.f; };
+            s_g4[k] = make_float4(g(r), g(r + 1), g(r + 2), g(r + 3));
+        }
+    }
     for (int k = threadIdx.x; k < N; k += blockDim.x) s_f[k] = a.use_filter ? a.filt2[k] : 1.0f;
     if (threadIdx.x == 0) {
         sfor<0, N>([&](auto kc) {
@@ -125,7 +161,7 @@ k_window_fp32(WinArgs a) {
         });
     }
     float2* buf = s_buf + team * S::BUF;
-    float* ab = reinterpret_cast<float*>(buf);  // |c|, after the last transform
+    float* ab = reinterpret_cast<float*>(buf);  // the correlation, after the last transform
     grid_dep_wait();  // the tables above come from the kernel's arguments
     const int nwork = *a.nwork;
     if (ln == 0) {
@@ -140,7 +176,8 @@ k_window_fp32(WinArgs a) {
         const bool valid = w < nwork;
         int gi = valid ? w : base;  // item index into work / peaks
         const float4* f12 = a.s12;
-        int nx = a.nx, ny = a.ny;
+        int nx = a.nx;
+        FastDiv ny = a.nyd;
         const float4* mp = a.means;
         MeanGrid mg = a.mg;
         if (a.nseg > 0) {
@@ -156,15 +193,15 @@ k_window_fp32(WinArgs a) {
         const int pix = a.work[gi];
         int i, j, imin, jmin;
         if (a.direct) {
-            imin = pix / ny;
+            imin = ny.div(pix);
             jmin = 0;
             i = imin;
             j = 0;
         } else {
-            i = pix / ny;
-            j = pix - i * ny;
+            i = ny.div(pix);
+            j = pix - i * ny.d;
             imin = box_start(i, nx, a.nsize);
-            jmin = box_start(j, ny, a.nsize);
+            jmin = box_start(j, ny.d, a.nsize);
         }
 
         // windowed, mean-subtracted column jj = ln of both frames: z = g1 + i g2
@@ -174,27 +211,46 @@ k_window_fp32(WinArgs a) {
                 (mp && !a.direct) ? __ldg(mp + mean_slot(mg, i, j)) : make_float4(0.f, 0.f, 0.f, 0.f);
             const float2 mh = make_float2(mm.x, mm.y), ml = make_float2(mm.z, mm.w);  // (f1, f2) hi, lo
             const float wc = s_g[ln + jmin - j + N];
-            const float4* p12 = f12 + (size_t)imin * ny + jmin + ln;
-            const float* gr = a.gauss + (imin - i + N);  // row weights: uniform, from the parameter bank
+            const float4* p12 = f12 + (size_t)imin * ny.d + jmin + ln;
             float mx1 = 0.f, mx2 = 0.f;
-            sfor<0, N>([&](auto ic) {
+            // (hi - mean hi) + (lo - mean lo) for both frames at once (packed
+            // f1/f2 pairs), both frames' pixel in one 16-byte load, times the
+            // separable weight; row ii goes where the column transform takes it
+            auto pixel = [&](auto ic, float g) {
                 constexpr int ii = decltype(ic)::value;
-                // (hi - mean hi) + (lo - mean lo) for both frames at once
-                // (packed f1/f2 pairs), both frames' pixel in one 16-byte load
-                const float4 q = __ldg(p12 + (size_t)ii * ny);
+                const float4 q = __ldg(p12 + (size_t)ii * ny.d);
                 const float2 dh = csub(make_float2(q.x, q.y), mh);
                 const float2 dl = csub(make_float2(q.z, q.w), ml);
-                const float wgt = wc * gr[ii];
-                const float2 z = cscale(cadd(dh, dl), wgt);
-                x[fft_in<N>(ii)] = z;  // row ii where the column transform takes it
-                mx1 = fmaxf(mx1, fabsf(z.x));
-                mx2 = fmaxf(mx2, fabsf(z.y));
-            });
+                const float2 z = cscale(cadd(dh, dl), wc * g);
+                x[fft_in<N>(ii)] = z;
+                return z;
+            };
+            if constexpr (kQuads) {
+                const int r0 = imin - i + N;  // weight index of the box's first row
+                const float4* gr = s_g4 + (r0 & 3) * (N / 2 + 1) + (r0 >> 2);
+                sfor<0, N / 4>([&](auto qc) {
+                    constexpr int q = 4 * decltype(qc)::value;
+                    const float4 g = gr[q / 4];
+                    const float2 z0 = pixel(std::integral_constant<int, q>{}, g.x);
+                    const float2 z1 = pixel(std::integral_constant<int, q + 1>{}, g.y);
+                    const float2 z2 = pixel(std::integral_constant<int, q + 2>{}, g.z);
+                    const float2 z3 = pixel(std::integral_constant<int, q + 3>{}, g.w);
+                    mx1 = max3_abs(max3_abs(mx1, z0.x, z1.x), z2.x, z3.x);
+                    mx2 = max3_abs(max3_abs(mx2, z0.y, z1.y), z2.y, z3.y);
+                });
+            } else {
+                const float* gr = a.gauss + (imin - i + N);  // row weights: uniform, from the parameter bank
+                sfor<0, N>([&](auto ic) {
+                    const float2 z = pixel(ic, gr[decltype(ic)::value]);
+                    mx1 = fmaxf(mx1, fabsf(z.x));
+                    mx2 = fmaxf(mx2, fabsf(z.y));
+                });
+            }
             unsigned b1, b2;
             if constexpr (kWarp) {
                 b1 = __reduce_max_sync(tmask, __float_as_uint(mx1));
                 b2 = __reduce_max_sync(tmask, __float_as_uint(mx2));
-                team_sync();  // the previous window's |c| reads are done
+                team_sync();  // the previous window's correlation is read
             } else {
                 atomicMax(&s_max[2 * team], __float_as_uint(mx1));
                 atomicMax(&s_max[2 * team + 1], __float_as_uint(mx2));
@@ -216,7 +272,7 @@ k_window_fp32(WinArgs a) {
         fft<N, 0, -1>(x);
         sfor<0, N>([&](auto kc) {
             constexpr int k = decltype(kc)::value;
-            buf[k * (N + 1) + ln] = x[fft_out<N>(k)];
+            buf[k * LD + ln] = x[fft_out<N>(k)];
         });
         team_sync();
         if constexpr (!kWarp) {
@@ -228,16 +284,25 @@ k_window_fp32(WinArgs a) {
                 s_key[team] = 0ull;
             }
         }
-        sfor<0, N>([&](auto jc) {
-            constexpr int jj = decltype(jc)::value;
-            x[fft_in<N>(jj)] = buf[ln * (N + 1) + jj];
-        });
+        if constexpr (kQuads) {
+            sfor<0, N / 2>([&](auto jc) {
+                constexpr int jj = 2 * decltype(jc)::value;
+                const float4 v = *reinterpret_cast<const float4*>(buf + ln * LD + jj);
+                x[fft_in<N>(jj)] = make_float2(v.x, v.y);
+                x[fft_in<N>(jj + 1)] = make_float2(v.z, v.w);
+            });
+        } else {
+            sfor<0, N>([&](auto jc) {
+                constexpr int jj = decltype(jc)::value;
+                x[fft_in<N>(jj)] = buf[ln * LD + jj];
+            });
+        }
         if constexpr (!kWarp) team_sync();
         fft<N, 0, -1>(x);  // thread ln now holds Z[kx = ln][ky] at x[fft_out<N>(ky)]
         if constexpr (!kWarp) {
             sfor<0, N>([&](auto kc) {
                 constexpr int k = decltype(kc)::value;
-                buf[ln * (N + 1) + k] = x[fft_out<N>(k)];
+                buf[ln * LD + k] = x[fft_out<N>(k)];
             });
             team_sync();
         }
@@ -266,7 +331,7 @@ k_window_fp32(WinArgs a) {
                     zm.x = __shfl_sync(tmask, x[fft_out<N>(mk)].x, mr, N);
                     zm.y = __shfl_sync(tmask, x[fft_out<N>(mk)].y, mr, N);
                 } else {
-                    zm = buf[mr * (N + 1) + mk];
+                    zm = buf[mr * LD + mk];
                 }
                 const float ax = z.x + zm.x, ay = z.y - zm.y;  // 2 s1 A
                 const float bx = z.y + zm.y, by = zm.x - z.x;  // 2 s2 B
@@ -289,12 +354,12 @@ k_window_fp32(WinArgs a) {
             } else if constexpr (kMirror) {
                 sfor<1, H>([&](auto kc) {
                     constexpr int k = decltype(kc)::value;
-                    buf[ln * (N + 1) + k] = y[k];
+                    buf[ln * LD + k] = y[k];
                 });
                 team_sync();
                 sfor<KC, N>([&](auto kc) {
                     constexpr int k = decltype(kc)::value;
-                    const float2 c = buf[mr * (N + 1) + (N - k)];
+                    const float2 c = buf[mr * LD + (N - k)];
                     y[k] = make_float2(c.x, -c.y);
                 });
             }
@@ -325,25 +390,49 @@ k_window_fp32(WinArgs a) {
             sfor<0, H>([&](auto mc) {
                 constexpr int m = decltype(mc)::value;
                 const float2 v = u[fft_out<H>(m)];
-                buf[ln * (N + 1) + m] = v;
-                buf[ln * (N + 1) + H + m] = make_float2(v.x * tw.x - v.y * tw.y, v.x * tw.y + v.y * tw.x);
+                buf[ln * LD + m] = v;
+                buf[ln * LD + H + m] = make_float2(v.x * tw.x - v.y * tw.y, v.x * tw.y + v.y * tw.x);
             });
         }
         team_sync();
         const int cm = ln % H, ch = ln / H;
         sfor<0, H>([&](auto kc) {
             constexpr int k = decltype(kc)::value;
-            u[fft_in<H>(k)] = cadd(buf[k * (N + 1) + ch * H + cm], buf[(k + H) * (N + 1) + ch * H + cm]);
+            u[fft_in<H>(k)] = cadd(buf[k * LD + ch * H + cm], buf[(k + H) * LD + ch * H + cm]);
         });
         fft<H, 0, +1>(u);  // u[fft_out<H>(i')] = c[2i'+h][2m] + i c[2i'+h][2m+1]
-        team_sync();  // |c| overwrites the transform buffer
+        team_sync();  // the correlation overwrites the transform buffer
 
-        unsigned long long key;  // max over the team of (|c|, -index)
-        // |c| in the half-shifted frame and the first strict maximum.  H is
-        // even, so the shifted row I = 2 I'' + h keeps the parity of i; a
-        // lane visits its values in increasing row-major order.
-        {
-            const int J = (2 * cm + H) % N;
+        // The correlation in the half-shifted frame and the first strict maximum
+        // of |c| (the least row-major index L that holds the largest value vb,
+        // as bits).  H is even, so the shifted row I = 2 I'' + h keeps the parity
+        // of i; a lane visits its values in increasing row-major order.
+        unsigned vb, L;
+        const int J = (2 * cm + H) % N;
+        if constexpr (kQuads) {
+            // largest value first, then its place: the team looks through the
+            // column pair of each lane that holds it (one, but for ties)
+            float bv = 0.f;
+            sfor<0, H>([&](auto Ic) {
+                constexpr int I2 = decltype(Ic)::value;
+                constexpr int ip = (I2 + H / 2) % H;
+                const float2 c = u[fft_out<H>(ip)];
+                *reinterpret_cast<float2*>(ab + (2 * I2 + ch) * N + J) = c;
+                bv = max3_abs(bv, c.x, c.y);
+            });
+            vb = __reduce_max_sync(tmask, __float_as_uint(bv));
+            unsigned win = __ballot_sync(0xffffffffu, __float_as_uint(bv) == vb) & tmask;
+            team_sync();
+            L = 0xffffffffu;
+            if (vb != 0u) {
+                for (; win; win &= win - 1u) {
+                    const int wl = (__ffs((int)win) - 1) & (N - 1);  // a holder's place in the team
+                    const int e = (2 * (ln >> 1) + wl / H) * N + (2 * (wl % H) + H) % N + (ln & 1);
+                    if (__float_as_uint(fabsf(ab[e])) == vb) L = min(L, (unsigned)e);
+                }
+            }
+            L = __reduce_min_sync(tmask, L);
+        } else {
             float bv = -1.0f;  // below every |c|; NaN never compares greater
             int bi = 0;        // row-major index of bv less ch * N + J
             sfor<0, H>([&](auto Ic) {
@@ -361,48 +450,50 @@ k_window_fp32(WinArgs a) {
                     bi = 2 * I2 * N + 1;
                 }
             });
-            // the team's maximum of (|c|, -index): the first strict maximum
+            // the team's maximum of (|c|, -index)
             const unsigned idx = (unsigned)(bi + ch * N + J);
             const unsigned khi = bv >= 0.0f ? __float_as_uint(bv) : 0u;
             const unsigned klo = bv >= 0.0f ? 0xffffffffu - idx : 0u;
             if constexpr (kWarp) {
-                const unsigned mhi = __reduce_max_sync(tmask, khi);
-                key = ((unsigned long long)mhi << 32) | __reduce_max_sync(tmask, khi == mhi ? klo : 0u);
+                vb = __reduce_max_sync(tmask, khi);
+                L = 0xffffffffu - __reduce_max_sync(tmask, khi == vb ? klo : 0u);
                 team_sync();
             } else {
                 atomicMax(&s_key[team], ((unsigned long long)khi << 32) | klo);
                 team_sync();
-                key = s_key[team];
+                const unsigned long long key = s_key[team];
+                vb = (unsigned)(key >> 32);
+                L = 0xffffffffu - (unsigned)key;
             }
         }
 
-        // integer peak (all lanes decode the same key), then the team stores
+        // integer peak (all lanes hold the same), then the team stores
         // the peak record for k_fit
         {
-            int I, J;
+            int I, Jp;
             bool have;
             const float v0 = ab[0];
             if (v0 != v0) {
                 // a NaN first element stays the maximum of a sequential scan
                 I = 0;
-                J = 0;
+                Jp = 0;
                 have = true;
             } else {
-                const unsigned L = 0xffffffffu - (unsigned)(key & 0xffffffffull);
-                have = __uint_as_float((unsigned)(key >> 32)) != 0.0f;
+                have = __uint_as_float(vb) != 0.0f;
                 I = have ? (int)(L / N) : N / 2;
-                J = have ? (int)(L % N) : N / 2;
+                Jp = have ? (int)(L % N) : N / 2;
             }
-            const bool dofit = have && I > 0 && I < N - 1 && J > 0 && J < N - 1;
+            const bool dofit = have && I > 0 && I < N - 1 && Jp > 0 && Jp < N - 1;
+            // kQuads left c itself in the buffer, the others |c|
             if (valid && a.peaks_h) {
                 // -h: the 6x6 patch around the peak, 37 words
                 float* rec = reinterpret_cast<float*>(a.peaks_h + gi);
                 for (int k = ln; k < kHiresPatch * kHiresPatch + 1; k += N) {
                     if (k < kHiresPatch * kHiresPatch) {
-                        const int r = I - 2 + k / kHiresPatch, c = J - 2 + k % kHiresPatch;
-                        rec[k] = (r >= 0 && r < N && c >= 0 && c < N) ? ab[r * N + c] : 0.f;
+                        const int r = I - 2 + k / kHiresPatch, c = Jp - 2 + k % kHiresPatch;
+                        rec[k] = (r >= 0 && r < N && c >= 0 && c < N) ? fabsf(ab[r * N + c]) : 0.f;
                     } else {
-                        rec[k] = __uint_as_float(peak_meta(I, J, have));
+                        rec[k] = __uint_as_float(peak_meta(I, Jp, have));
                     }
                 }
             } else if (valid) {
@@ -410,9 +501,9 @@ k_window_fp32(WinArgs a) {
                 float* rec = reinterpret_cast<float*>(a.peaks + gi);
                 for (int k = ln; k < 10; k += N) {
                     if (k < 9) {
-                        rec[k] = dofit ? ab[(I - 1 + k / 3) * N + (J - 1 + k % 3)] : 0.f;
+                        rec[k] = dofit ? fabsf(ab[(I - 1 + k / 3) * N + (Jp - 1 + k % 3)]) : 0.f;
                     } else {
-                        rec[9] = __uint_as_float(peak_meta(I, J, dofit));
+                        rec[9] = __uint_as_float(peak_meta(I, Jp, dofit));
                     }
                 }
             }

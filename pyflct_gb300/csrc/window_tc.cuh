@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(256, TcCfg<N>::MINB) k_window_tc(TcArgs a) {
             const WinSeg sg = a.segs[k];
             f.f12 = sg.s12;
             f.nx = sg.nx;
-            f.ny = sg.ny;
+            f.ny = sg.ny.d;
             if (mp) mp += sg.base;
             mg = sg.mg;
             w = sg.base + (w - __ldg(a.seg_start + k));
