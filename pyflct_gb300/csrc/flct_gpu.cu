@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "global.cuh"
+#include "host_copy.cuh"
 #include "prepass.cuh"
 #include "warp.cuh"
 #include "window_fp32.cuh"
@@ -167,6 +168,8 @@ struct flct_ctx {
     // computation: copy-in and copy-out streams, per-band events
     static constexpr int kMaxBands = 8;
     int host_bands_max = 5;        // FLCT_HOST_BANDS (0 or 1: one band)
+    bool host_bands_asked = false; // FLCT_HOST_BANDS is set
+    bool host_direct = false;      // the GPU may use pageable host addresses
     int host_bands = 0;            // bands of the pending host call (0: not banded)
     cudaStream_t cstream[2] = {};  // copy-in, copy-out
     // the prepass (highest priority) on three streams, classification, row
@@ -1973,8 +1976,17 @@ flct_status flct_gpu_create(int device, flct_ctx** out) {
         flct_gpu_destroy(ctx);
         return FLCT_ERR_CUDA;
     }
-    if (const char* nb = getenv("FLCT_HOST_BANDS"))
+    if (const char* nb = getenv("FLCT_HOST_BANDS")) {
         ctx->host_bands_max = std::max(0, std::min(flct_ctx::kMaxBands, atoi(nb)));
+        ctx->host_bands_asked = true;
+    }
+    {
+        int access = 0, tables = 0;
+        ctx->host_direct = cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, device) == cudaSuccess &&
+                           cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device) ==
+                               cudaSuccess &&
+                           access && tables;
+    }
     if (cudaHostAlloc((void**)&ctx->hctr, 64 * flct_ctx::kMaxBands, cudaHostAllocMapped) != cudaSuccess) {
         ctx->hctr = nullptr;
         flct_gpu_destroy(ctx);
@@ -2258,8 +2270,14 @@ flct_status flct_gpu_velocity(flct_ctx* ctx, const flct_params* p, const double*
     ENSURE(ctx->b_vm, npx * sizeof(double));
     cudaStream_t st = ctx->stream;
     // row bands whose copies overlap the computation, once the window form
-    // is settled (a first FLCT_FORM_AUTO call tunes in one band)
-    {
+    // is settled (a first FLCT_FORM_AUTO call tunes in one band).  Page-locked
+    // buffers only, where the bands are a replayed graph: the ~100 stream
+    // operations of an eager banded call cost more than their overlap gives
+    // (pageable, five bands against one: 201 x 101 362 against 147 us, 1024^2
+    // -s 4i 870 against 537, 1024^2 every pixel 3,727 against 3,004), unless
+    // FLCT_HOST_BANDS asks for them
+    const bool locked = page_locked(f1) && page_locked(f2) && page_locked(vx) && page_locked(vy) && page_locked(vm);
+    if (locked || ctx->host_bands_asked) {
         Job j;
         flct_status s = plan_job(ctx, p, (const double*)ctx->b_f1.p, (const double*)ctx->b_f2.p, nx, ny,
                                  (double*)ctx->b_vx.p, (double*)ctx->b_vy.p, (double*)ctx->b_vm.p, &j);
@@ -2283,8 +2301,11 @@ flct_status flct_gpu_velocity(flct_ctx* ctx, const flct_params* p, const double*
         }
     }
     CK(cudaEventRecord(ctx->ev[4], st));
-    CK(cudaMemcpyAsync(ctx->b_f1.p, f1, npx * sizeof(double), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(ctx->b_f2.p, f2, npx * sizeof(double), cudaMemcpyHostToDevice, st));
+    {
+        const double* src[] = {f1, f2};
+        double* dst[] = {(double*)ctx->b_f1.p, (double*)ctx->b_f2.p};
+        CK(copy_arrays(src, dst, 2, npx, cudaMemcpyHostToDevice, ctx->host_direct, st));
+    }
     CK(cudaEventRecord(ctx->ev[5], st));
     flct_status s = flct_gpu_velocity_device(ctx, p, (const double*)ctx->b_f1.p, (const double*)ctx->b_f2.p,
                                              nx, ny, (double*)ctx->b_vx.p, (double*)ctx->b_vy.p,
@@ -2293,9 +2314,13 @@ flct_status flct_gpu_velocity(flct_ctx* ctx, const flct_params* p, const double*
         cudaStreamSynchronize(st);
         return s;
     }
-    CK(cudaMemcpyAsync(vx, ctx->b_vx.p, nout * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(vy, ctx->b_vy.p, nout * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(vm, ctx->b_vm.p, nout * sizeof(double), cudaMemcpyDeviceToHost, st));
+    {
+        const double* src[] = {(const double*)ctx->b_vx.p, (const double*)ctx->b_vy.p, (const double*)ctx->b_vm.p};
+        double* dst[] = {vx, vy, vm};
+        if (!locked)
+            for (double* d : dst) populate_output(d, nout * sizeof(double));
+        CK(copy_arrays(src, dst, 3, (size_t)nout, cudaMemcpyDeviceToHost, ctx->host_direct, st));
+    }
     CK(cudaEventRecord(ctx->ev[6], st));
     CK(cudaStreamSynchronize(st));
     s = collect_timing(ctx);
@@ -2495,7 +2520,10 @@ flct_status flct_gpu_shift_frac2d(flct_ctx* ctx, const double* arr, double delx,
     // warp.c:811-820: shifts normalised by the axis lengths; transp swaps them
     const double dxarg = transp ? -dely / ((double)nx) : -delx / ((double)nx);
     const double dyarg = transp ? -delx / ((double)ny) : -dely / ((double)ny);
-    CK(cudaMemcpyAsync(ctx->b_f1.p, arr, n * sizeof(double), cudaMemcpyHostToDevice, st));
+    {
+        double* dst = (double*)ctx->b_f1.p;
+        CK(copy_arrays(&arr, &dst, 1, n, cudaMemcpyHostToDevice, ctx->host_direct, st));
+    }
     CK(cudaEventRecord(ctx->ev[0], st));
     if (fft) {
         // the same linear map by transforms, O(N log N)
@@ -2514,7 +2542,11 @@ flct_status flct_gpu_shift_frac2d(flct_ctx* ctx, const double* arr, double delx,
         CK(launch_real_part((const float2*)ctx->b_s2.p, (long)n, (double*)ctx->b_vx.p, st));
     }
     CK(cudaEventRecord(ctx->ev[1], st));
-    CK(cudaMemcpyAsync(out, ctx->b_vx.p, n * sizeof(double), cudaMemcpyDeviceToHost, st));
+    populate_output(out, n * sizeof(double));
+    {
+        const double* src = (const double*)ctx->b_vx.p;
+        CK(copy_arrays(&src, &out, 1, n, cudaMemcpyDeviceToHost, ctx->host_direct, st));
+    }
     CK(cudaStreamSynchronize(st));
     ctx->timing = flct_timing{};
     ctx->timing.launches = fft ? 5 + (ls.p[0].chirp || ls.p[1].chirp) : 7;
@@ -2543,9 +2575,11 @@ flct_status flct_gpu_warp_frac2d(flct_ctx* ctx, const double* arr, const double*
     ENSURE(ctx->b_aux1, fft ? line_setup_bytes(ls) : (size_t)(nx + ny) * sizeof(float2) + 64);
     float2* twx = (float2*)ctx->b_aux1.p;
     float2* twy = twx + nx;
-    CK(cudaMemcpyAsync(ctx->b_f1.p, arr, n * sizeof(double), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(ctx->b_f2.p, delx, n * sizeof(double), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(ctx->b_vy.p, dely, n * sizeof(double), cudaMemcpyHostToDevice, st));
+    {
+        const double* src[] = {arr, delx, dely};
+        double* dst[] = {(double*)ctx->b_f1.p, (double*)ctx->b_f2.p, (double*)ctx->b_vy.p};
+        CK(copy_arrays(src, dst, 3, n, cudaMemcpyHostToDevice, ctx->host_direct, st));
+    }
     CK(cudaEventRecord(ctx->ev[0], st));
     // F = forward DFT of the image (warp.c:899-934): transforms along both
     // axes where both have line plans, else DFT matrices
@@ -2578,7 +2612,11 @@ flct_status flct_gpu_warp_frac2d(flct_ctx* ctx, const double* arr, const double*
                            st));
     }
     CK(cudaEventRecord(ctx->ev[2], st));
-    CK(cudaMemcpyAsync(out, ctx->b_vx.p, n * sizeof(double), cudaMemcpyDeviceToHost, st));
+    populate_output(out, n * sizeof(double));
+    {
+        const double* src = (const double*)ctx->b_vx.p;
+        CK(copy_arrays(&src, &out, 1, n, cudaMemcpyDeviceToHost, ctx->host_direct, st));
+    }
     if (tc) CK(cudaMemcpyAsync(&wstatus, (unsigned*)ctx->b_wmisc.p + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     ctx->timing = flct_timing{};

@@ -1,0 +1,29 @@
+// host_copy.cuh -- copies between a caller's host arrays and the device for
+// the host-buffer entry points.
+#pragma once
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+namespace flct {
+
+// Arrays up to this size go in one kernel that reads or writes the host memory
+// itself, where the GPU shares the host's page tables: the rate is the copy
+// engine's (150-165 GB/s either way), and one launch replaces two to five
+// copies of about 10 us of latency each.  A call on 201 x 101 frames 147 ->
+// 105 us, 512^2 -s 3i 225 -> 178, 1024^2 -s 4i 532 -> 490.  Larger arrays
+// gain nothing by it, and pages that were never touched cost a kernel more
+// than the copy engine.
+constexpr size_t kHostKernelBytes = 1u << 24;
+
+// `count` arrays of n doubles, src[k] to dst[k], ordered on st.  direct: the
+// GPU may use pageable host addresses (cudaDevAttrPageableMemoryAccess with
+// the host's page tables).
+cudaError_t copy_arrays(const double* const* src, double* const* dst, int count, size_t n, cudaMemcpyKind kind,
+                        bool direct, cudaStream_t st);
+
+// Makes a caller's output pages present while the GPU computes: 8 MB of fresh
+// pages cost a copy 377 us through GPU faults, 52 us once they are there.
+// Leaves the contents as they are; errors are of no consequence.
+void populate_output(void* p, size_t bytes);
+
+}  // namespace flct
