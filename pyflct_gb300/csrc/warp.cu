@@ -221,18 +221,20 @@ __global__ void k_real_part(const float2* __restrict__ in, long n, double* __res
 // --------------------------------------------------------- warp sum ----
 
 // Per-pixel phase base in turns: ((double)idx - shift) / n, split hi + lo.
+// FP64 only for the difference and the product by 1 / n: conversions and
+// divisions run on the FP64 pipe too, which bounds this kernel (384 x 512:
+// 15 us with them).
 __global__ void k_warp_phase(const double* __restrict__ delx, const double* __restrict__ dely, int nx, int ny,
-                             int transp, float4* __restrict__ ph) {
+                             int transp, double inv_nx, double inv_ny, float4* __restrict__ ph) {
     const long n = (long)nx * ny;
     for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
         const int i = (int)(k / ny), j = (int)(k - (long)i * ny);
         // warp.c:948-959: transp swaps the roles of delx and dely
         const double sx = transp ? dely[k] : delx[k];
         const double sy = transp ? delx[k] : dely[k];
-        const double tx = (((double)i) - sx) / (double)nx;  // xarg / (2 pi)
-        const double ty = (((double)j) - sy) / (double)ny;
-        const float txh = (float)tx, tyh = (float)ty;
-        ph[k] = make_float4(txh, (float)(tx - (double)txh), tyh, (float)(ty - (double)tyh));
+        const float2 tx = split_double_fast(__dmul_rn(__dsub_rn(f2d((float)i), sx), inv_nx));  // xarg / (2 pi)
+        const float2 ty = split_double_fast(__dmul_rn(__dsub_rn(f2d((float)j), sy), inv_ny));
+        ph[k] = make_float4(tx.x, tx.y, ty.x, ty.y);
     }
 }
 
@@ -399,7 +401,7 @@ cudaError_t launch_real_part(const float2* in, long n, double* out, cudaStream_t
 cudaError_t launch_warp_phase(const double* delx, const double* dely, int nx, int ny, int transp, float4* ph,
                               cudaStream_t st) {
     const long n = (long)nx * ny;
-    k_warp_phase<<<(int)std::min<long>((n + 255) / 256, 4096), 256, 0, st>>>(delx, dely, nx, ny, transp, ph);
+    k_warp_phase<<<(int)std::min<long>((n + 255) / 256, 4096), 256, 0, st>>>(delx, dely, nx, ny, transp, 1.0 / nx, 1.0 / ny, ph);
     return cudaGetLastError();
 }
 

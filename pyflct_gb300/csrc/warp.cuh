@@ -29,11 +29,13 @@ cudaError_t launch_warp_phase(const double* delx, const double* dely, int nx, in
                               cudaStream_t st);
 cudaError_t launch_warp_sum(const float2* F, const float4* ph, int nx, int ny, double* out, cudaStream_t st);
 // the same sum on the tensor cores (split FP16, half spectrum): hs is
-// warp_tc_split_bytes(nx, ny) of scratch, misc two words (the spectrum's
-// largest |component| and the status word, misc[1]: kStatusTimeout bits);
-// stall_ns > 0 is a test hook (the first MMA wait gives up after stall_ns)
-size_t warp_tc_split_bytes(int nx, int ny);
+// warp_tc_split_bytes of scratch, misc warp_tc_misc_bytes of words (the
+// spectrum's largest |component|, the status word misc[1] with kStatusTimeout
+// bits, the tail groups' counts); nsm: the device's SMs; stall_ns > 0 is a
+// test hook (the first MMA wait gives up after stall_ns)
+size_t warp_tc_split_bytes(int nx, int ny, int nsm);
+size_t warp_tc_misc_bytes(int nsm);
 cudaError_t launch_warp_sum_tc(const float2* F, const float4* ph, int nx, int ny, void* hs, unsigned* misc,
-                               double* out, cudaStream_t st, unsigned long long stall_ns = 0);
+                               double* out, int nsm, cudaStream_t st, unsigned long long stall_ns = 0);
 
 }  // namespace flct

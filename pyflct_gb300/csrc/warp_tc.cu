@@ -30,14 +30,14 @@
 // stages of a chunk run from the highest columns down, each K step adds the
 // two cross products before hi*hi, and the DC term F[0][0] (the largest)
 // bypasses the GEMM and is added in FP64; the epilogue sums each 8-row
-// group in FP32 and the groups in FP64.
+// group in FP32 and the groups as float pairs (Sum2).
 //
 // CTA: 256 pixels (two 128-lane accumulators of 256 columns each, all 512
 // TMEM columns), 17 warps: warps 0-15 generate the A stages (two threads
 // per pixel, 8 columns each: exp(2 pi i c ty) as base(16 kc) x step(j),
-// both from exact float-float turn reductions), warps 0-7 also run the
-// epilogue of their own TMEM lane (row phases likewise as base x step per
-// 8 rows); lane 0 of warp 16 copies the pre-split B stages (one 32 KB bulk
+// both from exact float-float turn reductions) and run the epilogue of their
+// own TMEM lane, half a chunk's rows each (row phases likewise as base x step
+// per 8 rows); lane 0 of warp 16 copies the pre-split B stages (one 32 KB bulk
 // copy each) and issues the MMAs.  Three 64 KB stages in shared memory.  Every wait is
 // bounded (2 s); a wait that runs out sets the status word's timeout bit,
 // the CTA drains its own copies and MMAs (bounded), frees its tensor memory
@@ -79,34 +79,59 @@ __device__ __forceinline__ float wt_scale(unsigned maxbits) {
     return ldexpf(1.0f, max(-120, min(120, 14 - e)));
 }
 
+// Sum of floats kept as an unevaluated pair: every addition's rounding error
+// goes to the low part exactly, about 48 bits in all.  One FP64 addition (and
+// the conversion before it) holds the SM's FP64 pipe for 45 cycles a warp:
+// with FP64 sums the epilogue took 1,800 cycles per eight rows, most of it
+// there.
+struct Sum2 {
+    float hi = 0.0f, lo = 0.0f;
+    __device__ __forceinline__ void add(float b) {
+        const float s = __fadd_rn(hi, b), bb = __fsub_rn(s, hi);
+        lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bb)), __fsub_rn(b, bb)));
+        hi = s;
+    }
+    __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+};
+
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
 
-__device__ __forceinline__ unsigned h2_bits(__half2 h) {
-    return (unsigned)__half_as_ushort(__low2half(h)) | ((unsigned)__half_as_ushort(__high2half(h)) << 16);
-}
-
 // hi / lo FP16 halves of two values, packed (first value in the low half)
 __device__ __forceinline__ void split2(float v0, float v1, unsigned& hi, unsigned& lo) {
-    const __half2 h = __floats2half2_rn(v0, v1);
-    const float2 f = __half22float2(h);
-    hi = h2_bits(h);
-    lo = h2_bits(__floats2half2_rn(v0 - f.x, v1 - f.y));
+    float f0, f1;
+    asm("{\n.reg .b16 l, h;\ncvt.rn.f16x2.f32 %0, %4, %3;\nmov.b32 {l, h}, %0;\n"
+        "cvt.f32.f16 %1, l;\ncvt.f32.f16 %2, h;\n}"
+        : "=&r"(hi), "=&f"(f0), "=&f"(f1)
+        : "f"(v0), "f"(v1));
+    asm("cvt.rn.f16x2.f32 %0, %2, %1;" : "=r"(lo) : "f"(v0 - f0), "f"(v1 - f1));
+}
+
+__device__ __forceinline__ void st_shared16(uint32_t a, unsigned x, unsigned y, unsigned z, unsigned w) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(b)) : "memory");
 }
 
-// max |component| of the spectrum, as the bits of a non-negative float
-__global__ void k_wt_absmax(const float* __restrict__ f, long n, unsigned* __restrict__ mx) {
+// max |component| of the spectrum (n values, even), as the bits of a
+// non-negative float; NaN is passed over
+__global__ void __launch_bounds__(256) k_wt_absmax(const float2* __restrict__ f, long n2, unsigned* __restrict__ mx) {
+    __shared__ unsigned s_m[8];
     float m = 0.0f;
-    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x)
-        m = fmaxf(m, fabsf(f[k]));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(mx, __float_as_uint(m));
+    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n2; k += (long)gridDim.x * blockDim.x) {
+        const float2 v = f[k];
+        m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
+    }
+    const unsigned w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+    if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = w;
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        const unsigned b = __reduce_max_sync(0xffu, s_m[threadIdx.x]);
+        if (threadIdx.x == 0) atomicMax(mx, b);
+    }
 }
 
 // The B stages: block (q, kc) holds rows ii = 128 q .. +127 and columns
@@ -154,14 +179,17 @@ __global__ void k_wt_hsplit(const float2* __restrict__ F, int nx, int ny, int nk
 __global__ void __launch_bounds__(kWtThreads, 1)
     k_wt_sum(const unsigned char* __restrict__ hs, const float4* __restrict__ ph, const float2* __restrict__ F,
              const unsigned* __restrict__ mx, int nx, int ny, int nq, int nkc, double normfac,
-             double* __restrict__ out, unsigned* __restrict__ status, unsigned long long stall_ns) {
+             double* __restrict__ out, unsigned* __restrict__ status, unsigned long long stall_ns, int whole,
+             double* __restrict__ tail_part, unsigned* __restrict__ tail_count) {
     extern __shared__ unsigned char wt_raw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(wt_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     __shared__ __align__(8) uint64_t s_fa[kWtStages], s_fb[kWtStages], s_em[kWtStages];
     __shared__ __align__(8) uint64_t s_accf, s_acce, s_fin, s_never;  // s_never: test hook only
+    __shared__ double s_part[kWtPx];  // the sums over the upper half of each chunk's rows
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
+    __shared__ int s_last;
 
     const int t = threadIdx.x, w = t >> 5, lane = t & 31;
     if (t == 0) {
@@ -171,7 +199,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
             tc::mbar_init(&s_em[s], 1);
         }
         tc::mbar_init(&s_accf, 1);
-        tc::mbar_init(&s_acce, 8);
+        tc::mbar_init(&s_acce, kWtGen);
         tc::mbar_init(&s_fin, 1);
         tc::mbar_init(&s_never, 1);
         s_abort = 0;
@@ -183,7 +211,13 @@ __global__ void __launch_bounds__(kWtThreads, 1)
     tc::fence_after();
     const uint32_t tmem = s_tmem;
     const uint32_t sbase = tc::smem_u32(sm);
-    const int total = nq * nkc;
+    // the first `whole` CTAs take 256 pixels each, the others one 128-row chunk
+    // of the 256 pixels of their tail group
+    const int te = (int)blockIdx.x - whole;
+    const int qa = te >= 0 ? te % nq : 0, qn = te >= 0 ? 1 : nq;
+    const long px0 = (long)(te >= 0 ? whole + te / nq : (int)blockIdx.x) * kWtPx;
+    const int total = qn * nkc;
+    double sum = 0.0;  // this thread's share of its pixel
 
     // bounded wait; also gives up once another thread of the CTA has
     auto wait = [&](uint64_t* b, uint32_t par) -> bool {
@@ -215,7 +249,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
                 if (u > 0 && !wait(&s_em[s], (uint32_t)((u - 1) & 1))) return false;
                 tc::mbar_expect_tx(&s_fb[s], 2 * kWtBH);
                 const int q = g / nkc, kc = nkc - 1 - (g - q * nkc);
-                tc::bulk_g2s(sm + s * kWtStage + 4 * kWtAT, hs + ((size_t)q * nkc + kc) * (2 * kWtBH), 2 * kWtBH,
+                tc::bulk_g2s(sm + s * kWtStage + 4 * kWtAT, hs + ((size_t)(qa + q) * nkc + kc) * (2 * kWtBH), 2 * kWtBH,
                              &s_fb[s]);
                 return true;
             };
@@ -230,7 +264,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
                 s_abort = 1;
                 ok = false;
             }
-            for (int q = 0; q < nq && ok; ++q) {
+            for (int q = 0; q < qn && ok; ++q) {
                 if (q > 0) {
                     ok = wait(&s_acce, (uint32_t)((q - 1) & 1));
                     if (!ok) break;
@@ -275,21 +309,24 @@ __global__ void __launch_bounds__(kWtThreads, 1)
         __syncwarp();
     } else {
         // pixel t % 256 of the CTA; half h generates columns 8h .. 8h+7 of
-        // every stage; the threads of half 0 also run the epilogue (their
-        // warp w < 8 reads TMEM lane quadrant w % 4 of tile w / 4)
+        // every stage and sums rows 64h .. 64h+63 of every chunk (warp w reads
+        // TMEM lane quadrant w % 4 of tile (w / 4) % 2)
         const int pix = t & (kWtPx - 1), h = t / kWtPx;
         const int T = pix >> 7, m = pix & 127;
         const long npx = (long)nx * ny;
-        const long p = (long)blockIdx.x * kWtPx + pix;
+        const long p = px0 + pix;
         const bool live = p < npx;
         const float4 pb = live ? ph[p] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         const float sc = wt_scale(*mx);
         float2 S[8];  // exp(2 pi i (8h + j) ty), j < 8
 #pragma unroll
         for (int j = 0; j < 8; ++j) S[j] = turn_cs((float)(8 * h + j), pb.z, pb.w);
-        double acc = 0.0;
+        float2 Sx[8];  // exp(2 pi i j tx), j < 8
+#pragma unroll
+        for (int j = 0; j < 8; ++j) Sx[j] = turn_cs((float)j, pb.x, pb.y);
+        Sum2 acc;
         bool ok = true;
-        unsigned char* arow = sm + T * kWtAT + kmaj_off(m, 0);
+        const uint32_t arow = sbase + (uint32_t)(T * kWtAT + kmaj_off(m, 0) + h * 128);
         const uint32_t lane_base = (uint32_t)(32 * (w & 3)) << 16;
 
         auto epilogue = [&](int q) -> bool {
@@ -298,24 +335,28 @@ __global__ void __launch_bounds__(kWtThreads, 1)
             if (!__shfl_sync(0xffffffffu, done, 0)) return false;
             tc::fence_after();
             const uint32_t tb = tmem + lane_base + (uint32_t)(T * 256);
-            float2 Sx[8];  // exp(2 pi i j tx), j < 8
-#pragma unroll
-            for (int j = 0; j < 8; ++j) Sx[j] = turn_cs((float)j, pb.x, pb.y);
-#pragma unroll 1
-            for (int r0 = 0; r0 < 128; r0 += 8) {
-                const int i0 = q * 128 + r0;
-                if (i0 >= nx) break;
+            // eight rows at a time, the next eight on their way meanwhile
+            auto rows = [&](int i0, const uint32_t (&gr)[8], const uint32_t (&gi)[8]) {
+                if (i0 >= nx) return;
                 // rows i0 .. i0+7 have wavenumbers kx(i0) + j unless the
                 // wrap to negative wavenumbers falls inside the group
                 const bool run = i0 + 7 <= nx / 2 || i0 > nx / 2;
                 const float2 xb = turn_cs((float)freq_of(i0, nx), pb.x, pb.y);
-                float gr[8], gi[8];
-                tc::tmem_ld<8>(tb + r0, gr);
-                tc::tmem_ld<8>(tb + 128 + r0, gi);
                 float part = 0.0f;
+                if (run && i0 + 8 <= nx && (nx & 1 || nx / 2 < i0 || nx / 2 > i0 + 7)) {
+                    // no wrap, no end and no Nyquist row among the eight
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float2 ex = cmul(xb, Sx[j]);
+                        part = fmaf(ex.x, __uint_as_float(gr[j]), fmaf(-ex.y, __uint_as_float(gi[j]), part));
+                    }
+                    acc.add(part);
+                    return;
+                }
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     const int ii = i0 + j;
+                    const float re = __uint_as_float(gr[j]), im = __uint_as_float(gi[j]);
                     if (ii < nx) {
                         const float2 ex = run ? cmul(xb, Sx[j]) : turn_cs((float)freq_of(ii, nx), pb.x, pb.y);
                         if (2 * ii == nx) {
@@ -329,13 +370,32 @@ __global__ void __launch_bounds__(kWtThreads, 1)
                             }
                             a0.x *= sc;
                             a0.y *= sc;
-                            part += fmaf(ex.x, a0.x, -ex.y * a0.y) + 2.0f * ex.x * (gr[j] - a0.x);
+                            part += fmaf(ex.x, a0.x, -ex.y * a0.y) + 2.0f * ex.x * (re - a0.x);
                         } else {
-                            part = fmaf(ex.x, gr[j], fmaf(-ex.y, gi[j], part));
+                            part = fmaf(ex.x, re, fmaf(-ex.y, im, part));
                         }
                     }
                 }
-                acc += (double)part;
+                acc.add(part);
+            };
+            const int q0 = (qa + q) * 128 + 64 * h;
+            const uint32_t tr = tb + (uint32_t)(64 * h);
+            uint32_t ar[8], ai[8], br[8], bi[8];
+            tc::tmem_ld8_nw(tr, ar);
+            tc::tmem_ld8_nw(tr + 128, ai);
+            tc::tmem_wait_ld();
+#pragma unroll 1
+            for (int r0 = 0; r0 < 64; r0 += 16) {
+                tc::tmem_ld8_nw(tr + r0 + 8, br);
+                tc::tmem_ld8_nw(tr + 128 + r0 + 8, bi);
+                rows(q0 + r0, ar, ai);
+                tc::tmem_wait_ld();
+                if (r0 < 48) {
+                    tc::tmem_ld8_nw(tr + r0 + 16, ar);
+                    tc::tmem_ld8_nw(tr + 128 + r0 + 16, ai);
+                }
+                rows(q0 + r0 + 8, br, bi);
+                tc::tmem_wait_ld();
             }
             tc::fence_before();
             __syncwarp();
@@ -343,7 +403,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
             return true;
         };
 
-        for (int q = 0; q < nq && ok; ++q) {
+        for (int q = 0; q < qn && ok; ++q) {
             for (int kc = 0; kc < nkc && ok; ++kc) {
                 const int g = q * nkc + kc, s = g % kWtStages, u = g / kWtStages;
                 if (u > 0) {
@@ -354,7 +414,7 @@ __global__ void __launch_bounds__(kWtThreads, 1)
                 }
                 // stage kc of a chunk holds columns 16 (nkc - 1 - kc) .. +15
                 const float2 base = turn_cs((float)((nkc - 1 - kc) * 16), pb.z, pb.w);
-                unsigned char* dst = arow + s * kWtStage;
+                const uint32_t dst = arow + (uint32_t)(s * kWtStage);
                 unsigned rh[4], rl[4], ih[4], il[4];
 #pragma unroll
                 for (int e = 0; e < 8; e += 2) {
@@ -363,52 +423,99 @@ __global__ void __launch_bounds__(kWtThreads, 1)
                     split2(v0.x, v1.x, rh[e / 2], rl[e / 2]);
                     split2(v0.y, v1.y, ih[e / 2], il[e / 2]);
                 }
-                *reinterpret_cast<uint4*>(dst + h * 128) = make_uint4(rh[0], rh[1], rh[2], rh[3]);
-                *reinterpret_cast<uint4*>(dst + (2 + h) * 128) = make_uint4(ih[0], ih[1], ih[2], ih[3]);
-                *reinterpret_cast<uint4*>(dst + 2 * kWtAT + h * 128) = make_uint4(rl[0], rl[1], rl[2], rl[3]);
-                *reinterpret_cast<uint4*>(dst + 2 * kWtAT + (2 + h) * 128) = make_uint4(il[0], il[1], il[2], il[3]);
+                st_shared16(dst, rh[0], rh[1], rh[2], rh[3]);
+                st_shared16(dst + 2 * 128, ih[0], ih[1], ih[2], ih[3]);
+                st_shared16(dst + 2 * kWtAT, rl[0], rl[1], rl[2], rl[3]);
+                st_shared16(dst + 2 * kWtAT + 2 * 128, il[0], il[1], il[2], il[3]);
                 tc::fence_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&s_fa[s]);
                 // the previous chunk's epilogue, once this chunk's first
                 // stages are queued for the tensor cores
-                if (h == 0 && q > 0 && kc == (nkc > 1 ? 1 : 0)) ok = epilogue(q - 1);
+                if (q > 0 && kc == (nkc > 1 ? 1 : 0)) ok = epilogue(q - 1);
             }
         }
-        if (ok && h == 0) ok = epilogue(nq - 1);
-        if (ok && live && h == 0) out[p] = acc * (normfac / (double)sc) + (double)F[0].x * normfac;
+        if (ok) ok = epilogue(qn - 1);
+        sum = acc.value();
+        if (h) s_part[pix] = sum;
         if (!ok && lane == 0) atomicOr(status, kStatusTimeout);
     }
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
+    const long p = px0 + t;
+    const bool mine = t < kWtPx && p < (long)nx * ny;
+    if (te < 0) {
+        if (mine && !s_abort)
+            out[p] = (sum + s_part[t]) * (normfac / (double)wt_scale(*mx)) + (double)F[0].x * normfac;
+    } else if (!s_abort) {
+        // the last of a tail group's CTAs to arrive adds its chunks' sums in order
+        const int grp = te / nq;
+        double* const part = tail_part + (size_t)grp * nq * kWtPx;
+        if (t < kWtPx) part[(size_t)qa * kWtPx + t] = sum + s_part[t];
+        __threadfence();
+        __syncthreads();
+        if (t == 0) s_last = atomicAdd(tail_count + grp, 1u) == (unsigned)nq - 1u;
+        __syncthreads();
+        if (s_last && mine) {
+            __threadfence();
+            double v = 0.0;
+            for (int q = 0; q < nq; ++q) v += __ldcg(part + (size_t)q * kWtPx + t);
+            out[p] = v * (normfac / (double)wt_scale(*mx)) + (double)F[0].x * normfac;
+        }
+    }
     if (w == kWtGen) tc::tmem_dealloc(tmem, 512);
 }
 
 }  // namespace
 
-size_t warp_tc_split_bytes(int nx, int ny) {
-    const size_t nq = (size_t)(nx + 127) / 128, nkc = (size_t)(ny / 2 + 1 + 15) / 16;
-    return nq * nkc * (size_t)(2 * kWtBH);
+namespace {
+
+// CTAs of the sum: groups of 256 pixels, a whole one per CTA while they fill
+// every SM.  The groups left for the last round are cut into their row chunks
+// where that ends it sooner (tail x chunks CTAs of one chunk instead of tail
+// CTAs of all): 384 x 512 leaves 8 of 768 groups for a sixth round, 511 ->
+// 450 us.
+struct WtPlan {
+    int nq, nkc;
+    long groups, whole, tail;
+};
+WtPlan wt_plan(int nx, int ny, int nsm) {
+    WtPlan p{(nx + 127) / 128, (ny / 2 + 1 + 15) / 16, ((long)nx * ny + kWtPx - 1) / kWtPx, 0, 0};
+    p.tail = p.groups % nsm;
+    if ((p.tail * p.nq + nsm - 1) / nsm >= p.nq) p.tail = 0;
+    p.whole = p.groups - p.tail;
+    return p;
 }
 
+size_t stage_bytes(const WtPlan& p) { return (size_t)p.nq * p.nkc * (size_t)(2 * kWtBH); }
+
+}  // namespace
+
+size_t warp_tc_split_bytes(int nx, int ny, int nsm) {
+    const WtPlan p = wt_plan(nx, ny, nsm);
+    return stage_bytes(p) + (size_t)p.tail * p.nq * kWtPx * sizeof(double);
+}
+
+size_t warp_tc_misc_bytes(int nsm) { return (16 + (size_t)nsm) * sizeof(unsigned); }
+
 cudaError_t launch_warp_sum_tc(const float2* F, const float4* ph, int nx, int ny, void* hs, unsigned* misc,
-                               double* out, cudaStream_t st, unsigned long long stall_ns) {
-    const int nq = (nx + 127) / 128, nkc = (ny / 2 + 1 + 15) / 16;
+                               double* out, int nsm, cudaStream_t st, unsigned long long stall_ns) {
+    const WtPlan pl = wt_plan(nx, ny, nsm);
+    const int nq = pl.nq, nkc = pl.nkc;
     const long npx = (long)nx * ny;
-    cudaError_t e = cudaMemsetAsync(misc, 0, 2 * sizeof(unsigned), st);
+    cudaError_t e = cudaMemsetAsync(misc, 0, warp_tc_misc_bytes(nsm), st);
     if (e != cudaSuccess) return e;
-    const long nf = 2 * npx;
-    k_wt_absmax<<<(int)std::min<long>((nf + 255) / 256, 2048), 256, 0, st>>>(reinterpret_cast<const float*>(F), nf,
-                                                                             misc);
+    k_wt_absmax<<<(int)std::min<long>((npx + 255) / 256, 304), 256, 0, st>>>(F, npx, misc);
     const long nunits = (long)nq * nkc * 1024;
     k_wt_hsplit<<<(int)std::min<long>((nunits + 255) / 256, 65536), 256, 0, st>>>(F, nx, ny, nkc, nunits, misc,
                                                                                    reinterpret_cast<uint4*>(hs));
     e = cudaFuncSetAttribute(k_wt_sum, cudaFuncAttributeMaxDynamicSharedMemorySize, kWtSmem);
     if (e != cudaSuccess) return e;
-    k_wt_sum<<<(unsigned)((npx + kWtPx - 1) / kWtPx), kWtThreads, kWtSmem, st>>>(
-        reinterpret_cast<const unsigned char*>(hs), ph, F, misc, nx, ny, nq, nkc, 1.0 / (double)npx, out, misc + 1,
-        stall_ns);
+    unsigned char* const h = static_cast<unsigned char*>(hs);
+    k_wt_sum<<<(unsigned)(pl.whole + pl.tail * nq), kWtThreads, kWtSmem, st>>>(
+        h, ph, F, misc, nx, ny, nq, nkc, 1.0 / (double)npx, out, misc + 1, stall_ns, (int)pl.whole,
+        reinterpret_cast<double*>(h + stage_bytes(pl)), misc + 16);
     return cudaGetLastError();
 }
 
