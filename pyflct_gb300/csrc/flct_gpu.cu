@@ -747,12 +747,18 @@ BoxArgs box_rows_args(const Job& j, const JobBufs& b, int r0, int r1, long* task
 
 constexpr size_t kBoxRowsSmem = (size_t)kBoxWarps * (5 * (kRowSpan + 64) + 5 * 32) * sizeof(unsigned);
 
+// The column pass's run of grid rows (a property of the whole frame: its bands
+// use the same).
+bool long_runs(const Job& j) { return 2l * j.gi * j.gj >= kColLong; }
+int col_run(const Job& j) { return long_runs(j) ? kColRunLong : kColRun; }
+
 // Column pass arguments for grid rows [q0, q1), and its threads.
 BoxArgs box_cols_args(const Job& j, const JobBufs& b, int q0, int q1, long* threads) {
     BoxArgs ba = box_args(j, b);
     ba.q0 = q0;
     ba.q1 = q1;
-    *threads = 2l * j.gj * ((q1 - q0 + kColRun - 1) / kColRun) * kColLanes;
+    const int run = col_run(j);
+    *threads = 2l * j.gj * ((q1 - q0 + run - 1) / run) * (long_runs(j) ? 1 : kColLanes);
     return ba;
 }
 
@@ -776,13 +782,14 @@ flct_status enqueue_box_rows(flct_ctx* ctx, const Job& j, const JobBufs& b, int 
 }
 
 // Exact box sums of grid rows [q0, q1) (their row sums must be complete; q0
-// a multiple of kColRun, so the runs are those of the whole frame).
+// a multiple of col_run, so the runs are those of the whole frame).
 flct_status enqueue_box_cols(flct_ctx* ctx, const Job& j, const JobBufs& b, int q0, int q1, cudaStream_t st,
                              int* launches, bool pdl = false) {
     if (q1 <= q0) return FLCT_OK;
     long t = 0;
     BoxArgs ba = box_cols_args(j, b, q0, q1, &t);
-    CK(launch_kernel(k_box_cols, dim3((unsigned)((t + 127) / 128)), dim3(128), 0, st, pdl, ba));
+    CK(launch_kernel(long_runs(j) ? k_box_cols_long : k_box_cols, dim3((unsigned)((t + 127) / 128)), dim3(128), 0, st,
+                     pdl, ba));
     ++*launches;
     CK(cudaGetLastError());
     return FLCT_OK;
@@ -1108,7 +1115,7 @@ struct BatchPlan {
     std::vector<Job> jobs;
     std::vector<JobBufs> bufs;
     std::vector<BatchGroup> groups;
-    MultiSet m_abs, m_thr, m_cls, m_rows, m_cols, m_fit, m_fith, m_interp;
+    MultiSet m_abs, m_thr, m_cls, m_rows, m_cols, m_colsl, m_fit, m_fith, m_interp;
     WinSeg* segs = nullptr;  // device, group-major
     int* starts = nullptr;   // device, per group nseg + 1 entries
     int* seg_pair = nullptr; // device
@@ -1183,7 +1190,7 @@ flct_status plan_multi(flct_ctx* ctx, BatchPlan* bp) {
     std::vector<BoxArgs> rows, cols;
     std::vector<FitArgs> fit, fith;
     std::vector<InterpArgs> ia;
-    std::vector<long> babs, bthr, bcls, brows, bcols, bfit, bfith, bia;
+    std::vector<long> babs, bthr, bcls, brows, bcols, bcolsl, bfit, bfith, bia;
     for (int k = 0; k < np; ++k) {
         const Job& j = bp->jobs[k];
         const JobBufs& b = bp->bufs[k];
@@ -1200,7 +1207,8 @@ flct_status plan_multi(flct_ctx* ctx, BatchPlan* bp) {
         rows.push_back(box_rows_args(j, b, 0, j.nx, &tasks));
         brows.push_back((tasks + kBoxWarps - 1) / kBoxWarps);
         cols.push_back(box_cols_args(j, b, 0, j.gi, &threads));
-        bcols.push_back((threads + 127) / 128);
+        bcols.push_back(long_runs(j) ? 0 : (threads + 127) / 128);
+        bcolsl.push_back(long_runs(j) ? (threads + 127) / 128 : 0);
         const FitArgs fa = fit_args(j, b, Pub{});
         fit.push_back(fa);
         fith.push_back(fa);
@@ -1209,7 +1217,7 @@ flct_status plan_multi(flct_ctx* ctx, BatchPlan* bp) {
         ia.push_back(interp_args(j, b, 0, j.nx, Pub{}));
         bia.push_back(j.interp ? (long)((j.nx + kTileR - 1) / kTileR) * ((j.ny + kTileC - 1) / kTileC) : 0);
     }
-    for (const auto* v : {&babs, &bthr, &bcls, &brows, &bcols, &bfit, &bfith, &bia}) {
+    for (const auto* v : {&babs, &bthr, &bcls, &brows, &bcols, &bcolsl, &bfit, &bfith, &bia}) {
         long tot = 0;
         for (long x : *v) tot += x;
         if (tot >= (1l << 31)) return fail(ctx, FLCT_ERR_UNSUPPORTED, "batch needs more than 2^31 blocks");
@@ -1219,6 +1227,7 @@ flct_status plan_multi(flct_ctx* ctx, BatchPlan* bp) {
     pack(cls, bcls, &bp->m_cls);
     pack(rows, brows, &bp->m_rows);
     pack(cols, bcols, &bp->m_cols);
+    pack(cols, bcolsl, &bp->m_colsl);
     pack(fit, bfit, &bp->m_fit);
     pack(fith, bfith, &bp->m_fith);
     pack(ia, bia, &bp->m_interp);
@@ -1410,6 +1419,7 @@ flct_status enqueue_batch_prepass(flct_ctx* ctx, BatchPlan& bp, cudaStream_t bs,
     CK(launch_multi(ctx, k_box_rows_multi, bp.m_rows, kBoxWarps * 32, kBoxRowsSmem, bs, launches));
     CK(launch_multi(ctx, k_classify_multi, bp.m_cls, 256, 0, cs, launches));
     CK(launch_multi(ctx, k_box_cols_multi, bp.m_cols, 128, 0, bs, launches));
+    CK(launch_multi(ctx, k_box_cols_long_multi, bp.m_colsl, 128, 0, bs, launches));
     if (side) {
         CK(cudaEventRecord(ctx->bev[1], side));
         CK(cudaStreamWaitEvent(bs, ctx->bev[1], 0));
@@ -1608,11 +1618,12 @@ struct Bands {
 
 bool plan_bands(const flct_ctx* ctx, const Job& j, Bands* bd) {
     if (j.d.global || j.d.rel_thresh || j.gi < 1) return false;
-    for (int nb = std::min(ctx->host_bands_max, j.gi / (2 * kColRun)); nb >= 2; --nb) {
+    const int run = col_run(j);
+    for (int nb = std::min(ctx->host_bands_max, j.gi / (2 * run)); nb >= 2; --nb) {
         bool ok = true;
         // band starts at multiples of the column pass's run
         for (int b = 0; b <= nb; ++b)
-            bd->Q[b] = (b == nb) ? j.gi : (int)((long)j.gi * b / nb) / kColRun * kColRun;
+            bd->Q[b] = (b == nb) ? j.gi : (int)((long)j.gi * b / nb) / run * run;
         for (int b = 0; b <= nb; ++b) bd->R[b] = (b == 0) ? 0 : (b == nb) ? j.nx : j.xo + bd->Q[b] * j.gs;
         bd->O[0] = 0;
         bd->O[nb] = j.nx;

@@ -317,63 +317,49 @@ __device__ __forceinline__ void k_box_rows_body(const BoxArgs& a, const int vb, 
 FLCT_MULTI_KERNEL(__launch_bounds__(kBoxWarps * 32), k_box_rows, BoxArgs)
 
 // Box sums B[q][m] = sum_{ii<n} RT[t_q + ii][m] at the grid's box rows
-// t_q = box_start(xo + q gs), exact.  kColLanes consecutive lanes take one
-// line (frame, grid column) and a run of kColRun grid rows starting at a
-// multiple of kColRun; lane p reads the run's rows r with r - t = p mod
-// kColLanes, and the lanes' partial sums meet by shuffles (integer sums:
-// the order does not matter).  The run's unit is the largest of the row
-// sums' units it reads.  A warp's loads cover 32 / kColLanes consecutive
-// columns of kColLanes rows.  Each box sum becomes the grid point's FP64
+// t_q = box_start(xo + q gs), exact.  LANES consecutive lanes take one line
+// (frame, grid column) and a run of grid rows starting at a multiple of the
+// run's length (kColRun with kColLanes lanes, kColRunLong with one); lane p
+// reads the run's rows r with r - t = p mod LANES, and the lanes' partial
+// sums meet by shuffles (integer sums: the order does not matter).  The
+// run's unit is the largest of the row sums' units it reads.  A warp's loads
+// cover 32 / LANES consecutive columns of LANES rows.  Each box sum becomes the grid point's FP64
 // local mean, rounded once, and is stored as its float hi + lo split (the
 // form the window kernels subtract): lane 0 of the group writes this
 // frame's half of the grid point's float4.
+template <int LANES>
 __device__ __forceinline__ void col_reduce(unsigned long long& lo, unsigned long long& hi,
                                            unsigned long long& cnt) {
 #pragma unroll
-    for (int o = 1; o < kColLanes; o <<= 1) {
-        const unsigned long long l2 = __shfl_xor_sync(0xffffffffu, lo, o, kColLanes);
-        const unsigned long long h2 = __shfl_xor_sync(0xffffffffu, hi, o, kColLanes);
-        cnt += __shfl_xor_sync(0xffffffffu, cnt, o, kColLanes);
+    for (int o = 1; o < LANES; o <<= 1) {
+        const unsigned long long l2 = __shfl_xor_sync(0xffffffffu, lo, o, LANES);
+        const unsigned long long h2 = __shfl_xor_sync(0xffffffffu, hi, o, LANES);
+        cnt += __shfl_xor_sync(0xffffffffu, cnt, o, LANES);
         add128(lo, hi, l2, h2);
     }
 }
 
-__device__ __forceinline__ void k_box_cols_body(const BoxArgs& a, const int vb, const int vg) {
-    grid_dep_wait();  // the row sums come from the kernel before
-    const int lines = 2 * a.gj;
-    const int runs = (a.q1 - a.q0 + kColRun - 1) / kColRun;
-    const long gid = vb * (long)blockDim.x + threadIdx.x;
-    const int p = (int)(gid & (kColLanes - 1));
-    long idx = gid / kColLanes;
-    // a group past the end repeats the last line (every lane of the warp
-    // takes part in the shuffles) and stores nothing
-    const bool act = idx < (long)lines * runs;
-    if (!act) idx = (long)lines * runs - 1;
-    const int run = (int)(idx / lines), lam = (int)(idx - (long)run * lines);
-    const int img = lam >= a.gj, m = lam - img * a.gj;
-    const BoxSum* __restrict__ v = (img ? a.rt2 : a.rt1) + m;  // row r at v[r * gj]
-    const int* __restrict__ ve = (img ? a.re2 : a.re1) + m;
-    // this line's hi and lo in the grid points' float4 means (f1 hi, f2 hi,
-    // f1 lo, f2 lo): floats img and 2 + img
-    float* __restrict__ o = reinterpret_cast<float*>(a.means + m) + img;
-    const size_t gj = (size_t)a.gj;
-    const int q0 = a.q0 + run * kColRun, q1 = min(q0 + kColRun, a.q1);
+// Grid rows [q0, q1) of one line: v and ve the line's row sums and their
+// exponents (row r at r gj), o its floats in the means.
+template <int LANES>
+__device__ __forceinline__ void box_run(const BoxArgs& a, const BoxSum* __restrict__ v, const int* __restrict__ ve,
+                                        float* __restrict__ o, size_t gj, int q0, int q1, int p, bool act) {
     int t = box_start(a.xo + q0 * a.gs, a.nx, a.nsize);
     const int tend = box_start(a.xo + (q1 - 1) * a.gs, a.nx, a.nsize) + a.n;
     int eb = 1;
 #pragma unroll 4
-    for (int r = t + p; r < tend; r += kColLanes) eb = max(eb, __ldg(ve + r * gj));
+    for (int r = t + p; r < tend; r += LANES) eb = max(eb, __ldg(ve + r * gj));
 #pragma unroll
-    for (int k = 1; k < kColLanes; k <<= 1) eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, k, kColLanes));
+    for (int k = 1; k < LANES; k <<= 1) eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, k, LANES));
     unsigned long long lo = 0ull, hi = 0ull, cnt = 0ull;
 #pragma unroll 8
-    for (int r = t + p; r < t + a.n; r += kColLanes) {
+    for (int r = t + p; r < t + a.n; r += LANES) {
         BoxSum x = v[r * gj];
         sar128(x.lo, x.hi, eb - (int)x.e);
         add128(lo, hi, x.lo, x.hi);
         cnt += x.cnt;
     }
-    col_reduce(lo, hi, cnt);
+    col_reduce<LANES>(lo, hi, cnt);
     for (int q = q0;;) {
         if (act && p == 0) {
             // the FP64 mean (flct.c:815-827), rounded once from the exact sum
@@ -388,7 +374,7 @@ __device__ __forceinline__ void k_box_cols_body(const BoxArgs& a, const int vb, 
         const int tn = box_start(a.xo + q * a.gs, a.nx, a.nsize);
         unsigned long long dl = 0ull, dh = 0ull, dc = 0ull;
 #pragma unroll 2
-        for (int r = t + p; r < tn; r += kColLanes) {
+        for (int r = t + p; r < tn; r += LANES) {
             BoxSum in = v[(r + a.n) * gj], out = v[r * gj];
             sar128(in.lo, in.hi, eb - (int)in.e);
             sar128(out.lo, out.hi, eb - (int)out.e);
@@ -396,13 +382,64 @@ __device__ __forceinline__ void k_box_cols_body(const BoxArgs& a, const int vb, 
             sub128(dl, dh, out.lo, out.hi);
             dc += in.cnt - out.cnt;
         }
-        col_reduce(dl, dh, dc);
+        col_reduce<LANES>(dl, dh, dc);
         add128(lo, hi, dl, dh);
         cnt += dc;
         t = tn;
     }
 }
+
+template <int LANES>
+__device__ __forceinline__ void box_cols(const BoxArgs& a, const int vb) {
+    constexpr int RUN = LANES == 1 ? kColRunLong : kColRun;
+    const int lines = 2 * a.gj;
+    const int runs = (a.q1 - a.q0 + RUN - 1) / RUN;
+    const long gid = vb * (long)blockDim.x + threadIdx.x;
+    const int p = (int)(gid & (LANES - 1));
+    long idx = gid / LANES;
+    // a group past the end repeats the last line (every lane of the warp
+    // takes part in the shuffles) and stores nothing
+    const bool act = idx < (long)lines * runs;
+    if (!act) idx = (long)lines * runs - 1;
+    const int run = (int)(idx / lines), lam = (int)(idx - (long)run * lines);
+    const int img = lam >= a.gj, m = lam - img * a.gj;
+    const BoxSum* __restrict__ v = (img ? a.rt2 : a.rt1) + m;  // row r at v[r * gj]
+    const int* __restrict__ ve = (img ? a.re2 : a.re1) + m;
+    // this line's hi and lo in the grid points' float4 means (f1 hi, f2 hi,
+    // f1 lo, f2 lo): floats img and 2 + img
+    float* __restrict__ o = reinterpret_cast<float*>(a.means + m) + img;
+    const size_t gj = (size_t)a.gj;
+    const int q0 = a.q0 + run * RUN, q1 = min(q0 + RUN, a.q1);
+    if constexpr (LANES == 1) {
+        // a long run whose rows' units lie far apart goes in pieces of kColRun,
+        // so that its small boxes keep the unit a short run gives them
+        const int t0 = box_start(a.xo + q0 * a.gs, a.nx, a.nsize);
+        const int t1 = box_start(a.xo + (q1 - 1) * a.gs, a.nx, a.nsize) + a.n;
+        int emax = 1, emin = 0x7fffffff;
+#pragma unroll 4
+        for (int r = t0; r < t1; ++r) {
+            const int e = __ldg(ve + r * gj);
+            emax = max(emax, e);
+            emin = min(emin, e);
+        }
+        const int piece = emax - emin > 8 ? kColRun : RUN;
+        for (int q = q0; q < q1; q += piece) box_run<1>(a, v, ve, o, gj, q, min(q + piece, q1), p, act);
+    } else {
+        box_run<LANES>(a, v, ve, o, gj, q0, q1, p, act);
+    }
+}
+
+__device__ __forceinline__ void k_box_cols_body(const BoxArgs& a, const int vb, const int) {
+    grid_dep_wait();  // the row sums come from the kernel before
+    box_cols<kColLanes>(a, vb);
+}
 FLCT_MULTI_KERNEL(__launch_bounds__(128), k_box_cols, BoxArgs)
+
+__device__ __forceinline__ void k_box_cols_long_body(const BoxArgs& a, const int vb, const int) {
+    grid_dep_wait();
+    box_cols<1>(a, vb);
+}
+FLCT_MULTI_KERNEL(__launch_bounds__(128), k_box_cols_long, BoxArgs)
 
 // --------------------------------------------------- interpolation ----
 

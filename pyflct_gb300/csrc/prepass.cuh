@@ -32,11 +32,18 @@ constexpr int kClassPix = 256 * kClassPpt;
 // warp converts into shared memory per pass.
 constexpr int kBoxWarps = 4;
 constexpr int kRowSpan = 544;
-// Column pass: grid rows per thread, runs start at multiples of it (the
-// units of a run's box sums depend on the rows it reads)
-constexpr int kColRun = 4;
-// Column pass: lanes that share one run's rows (a power of two <= 32)
-constexpr int kColLanes = 4;
+// Column pass: runs of grid rows, starting at multiples of their length (the
+// units of a run's box sums depend on the rows it reads).  Small grids want
+// short chains: four lanes share a run of four.  From kColLong grid points
+// (both frames) on there are lanes enough, and a lane of its own per run of 16
+// reads each row sum (n + 15) / 16 times instead of (n + 3) / 4.  Prepass of
+// 2048^2 -s 2 at box 64 265 -> 187 us, 769 x 1023 every pixel at box 48 152 ->
+// 80, 1500 x 1800 at box 12 317 -> 163; at 524,288 points (512^2 every pixel,
+// box 32) 46 against 45, at 131,072 (1024^2 -s 4) 36 against 75.  Two kernels,
+// as one with both branches costs the small grids 0.5-1 us of code.
+constexpr int kColRun = 4, kColLanes = 4;
+constexpr int kColRunLong = 16;
+constexpr long kColLong = 800000;
 
 // Local means for the boxes the grid needs, from exact box sums
 // (fixsum.cuh).  Grid point (q, m) is pixel (xo + q gs, yo + m gs) (gs = 1,
@@ -92,12 +99,14 @@ __global__ void k_thresh_final(ThreshArgs a);
 __global__ void k_classify(ClassifyArgs a);
 __global__ void k_box_rows(BoxArgs a);
 __global__ void k_box_cols(BoxArgs a);
+__global__ void k_box_cols_long(BoxArgs a);
 // the same kernels over many frame pairs at once (MultiArgs, common.cuh)
 __global__ void k_absmax_multi(MultiArgs<AbsmaxArgs> m);
 __global__ void k_thresh_final_multi(MultiArgs<ThreshArgs> m);
 __global__ void k_classify_multi(MultiArgs<ClassifyArgs> m);
 __global__ void k_box_rows_multi(MultiArgs<BoxArgs> m);
 __global__ void k_box_cols_multi(MultiArgs<BoxArgs> m);
+__global__ void k_box_cols_long_multi(MultiArgs<BoxArgs> m);
 __global__ void k_interp_grid_multi(MultiArgs<InterpArgs> m);
 __global__ void k_interp_axis(int n, int gcount, int off, int skip, const double* want, int* zero,
                               double* wts, unsigned char* ok);
