@@ -1,4 +1,8 @@
-"""The column pass's long runs (large grids): velocities against the oracle on\nsampled pixels, with flat frames and with frames whose values change by\ndecades row by row, and bands of a host call against one band.  Grids on both\nsides of the rule's line (800,000 points of both frames)."""
+"""The column pass's long runs (large grids): velocities against the oracle on
+sampled pixels, with flat frames and with frames whose values change by
+decades row by row, and bands of a host call against one band.  Grids on both
+sides of the rule's line (800,000 points of both frames)."""
+import ctypes as C
 
 import numpy as np
 import pytest
