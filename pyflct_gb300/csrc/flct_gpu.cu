@@ -749,7 +749,7 @@ constexpr size_t kBoxRowsSmem = (size_t)kBoxWarps * (5 * (kRowSpan + 64) + 5 * 3
 
 // The column pass's run of grid rows (a property of the whole frame: its bands
 // use the same).
-bool long_runs(const Job& j) { return 2l * j.gi * j.gj >= kColLong; }
+bool long_runs(const Job& j) { return 4l * j.gi * j.gj >= kColLong * (j.gs + 1); }
 int col_run(const Job& j) { return long_runs(j) ? kColRunLong : kColRun; }
 
 // Column pass arguments for grid rows [q0, q1), and its threads.

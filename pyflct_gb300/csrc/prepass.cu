@@ -339,27 +339,98 @@ __device__ __forceinline__ void col_reduce(unsigned long long& lo, unsigned long
     }
 }
 
-// Grid rows [q0, q1) of one line: v and ve the line's row sums and their
-// exponents (row r at r gj), o its floats in the means.
+// The largest (and smallest) exponent of rows t + p, t + p + LANES, .. below
+// tend, U loads in flight whatever the count.
 template <int LANES>
-__device__ __forceinline__ void box_run(const BoxArgs& a, const BoxSum* __restrict__ v, const int* __restrict__ ve,
-                                        float* __restrict__ o, size_t gj, int q0, int q1, int p, bool act) {
-    int t = box_start(a.xo + q0 * a.gs, a.nx, a.nsize);
-    const int tend = box_start(a.xo + (q1 - 1) * a.gs, a.nx, a.nsize) + a.n;
-    int eb = 1;
-#pragma unroll 4
-    for (int r = t + p; r < tend; r += LANES) eb = max(eb, __ldg(ve + r * gj));
+__device__ __forceinline__ void exp_range(const int* __restrict__ ve, size_t gj, int t, int tend, int& emax, int& emin) {
+    constexpr int U = LANES > 1 ? 12 : 4;
+    for (int r0 = t; r0 < tend; r0 += U * LANES) {
+        int e[U];
 #pragma unroll
-    for (int k = 1; k < LANES; k <<= 1) eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, k, LANES));
+        for (int u = 0; u < U; ++u) e[u] = r0 + u * LANES < tend ? __ldg(ve + (r0 + u * LANES) * gj) : 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            emax = max(emax, e[u]);
+            if (r0 + u * LANES < tend) emin = min(emin, e[u]);
+        }
+    }
+}
+
+// Rows r = r0, r0 + LANES, .. below r1 added to an exact sum in units of eb,
+// U loads in flight whatever the count (a loop unrolled the plain way takes
+// its remainder one round trip a row).
+template <int LANES>
+__device__ __forceinline__ void add_rows(const BoxSum* __restrict__ v, size_t gj, int r0, int r1, int eb,
+                                         unsigned long long& lo, unsigned long long& hi, unsigned long long& cnt) {
+    constexpr int U = LANES > 1 ? 4 : 3;  // long runs: 1500 x 1800 at box 12 157 us, 165 with 4
+    for (; r0 < r1; r0 += U * LANES) {
+        BoxSum x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            x[u] = BoxSum{0ull, 0ull, 0ull, 0ull};
+            if (r0 + u * LANES < r1) x[u] = v[(r0 + u * LANES) * gj];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            sar128(x[u].lo, x[u].hi, eb - (int)x[u].e);
+            add128(lo, hi, x[u].lo, x[u].hi);
+            cnt += x[u].cnt;
+        }
+    }
+}
+
+// Grid rows [q0, q1) of one line: v the line's row sums (row r at r gj), eb
+// the run's unit, o its floats in the means.  What bounds a short run is its
+// chain of loads (0.2 waves of blocks): one round trip for the exponents, one
+// for 16 rows of the first box, one for those of all slides.  Prepass with the
+// rows loaded as they are needed -> now: 128^2 at box 16 15.4 -> 14.3 us, 201 x
+// 101 at box 20 16.3 -> 15.3, 512^2 -s 4 at box 32 22 -> 18.7.
+template <int LANES>
+__device__ __forceinline__ void box_run(const BoxArgs& a, const BoxSum* __restrict__ v, float* __restrict__ o, size_t gj,
+                                        int q0, int q1, int p, bool act, int eb) {
+    auto start = [&](int q) { return box_start(a.xo + q * a.gs, a.nx, a.nsize); };
+    // slide from the box at row t0 to the one at t1: rows [t0, t1) leave,
+    // rows [t0 + n, t1 + n) enter
+    struct Delta {
+        unsigned long long lo, hi, cnt;
+    };
+    auto slide = [&](Delta& d, BoxSum in, BoxSum out) {
+        sar128(in.lo, in.hi, eb - (int)in.e);
+        sar128(out.lo, out.hi, eb - (int)out.e);
+        add128(d.lo, d.hi, in.lo, in.hi);
+        sub128(d.lo, d.hi, out.lo, out.hi);
+        d.cnt += in.cnt - out.cnt;
+    };
+    int t = start(q0);
     unsigned long long lo = 0ull, hi = 0ull, cnt = 0ull;
-#pragma unroll 8
-    for (int r = t + p; r < t + a.n; r += LANES) {
-        BoxSum x = v[r * gj];
-        sar128(x.lo, x.hi, eb - (int)x.e);
-        add128(lo, hi, x.lo, x.hi);
-        cnt += x.cnt;
+    add_rows<LANES>(v, gj, t + p, t + a.n, eb, lo, hi, cnt);
+    constexpr int AHEAD = LANES > 1 ? kColRun - 1 : 1;
+    Delta dk[AHEAD];
+    if constexpr (LANES > 1) {
+        BoxSum in[AHEAD], out[AHEAD];
+        int tk = t;
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k) {
+            const int tn = q0 + 1 + k < q1 ? start(q0 + 1 + k) : tk;
+            in[k] = out[k] = BoxSum{0ull, 0ull, 0ull, 0ull};
+            if (tk + p < tn) {
+                in[k] = v[(tk + p + a.n) * gj];
+                out[k] = v[(tk + p) * gj];
+            }
+            tk = tn;
+        }
+        tk = t;
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k) {
+            const int tn = q0 + 1 + k < q1 ? start(q0 + 1 + k) : tk;
+            dk[k] = Delta{0ull, 0ull, 0ull};
+            slide(dk[k], in[k], out[k]);
+            for (int r = tk + p + LANES; r < tn; r += LANES) slide(dk[k], v[(r + a.n) * gj], v[r * gj]);
+            tk = tn;
+        }
     }
     col_reduce<LANES>(lo, hi, cnt);
+#pragma unroll 1
     for (int q = q0;;) {
         if (act && p == 0) {
             // the FP64 mean (flct.c:815-827), rounded once from the exact sum
@@ -369,23 +440,20 @@ __device__ __forceinline__ void box_run(const BoxArgs& a, const BoxSum* __restri
             o[(size_t)q * gj * 4 + 2] = mhl.y;
         }
         if (++q >= q1) break;
-        // slide down to the next grid row's box: rows [t, tn) leave, rows
-        // [t + n, tn + n) enter
-        const int tn = box_start(a.xo + q * a.gs, a.nx, a.nsize);
-        unsigned long long dl = 0ull, dh = 0ull, dc = 0ull;
+        Delta d = Delta{0ull, 0ull, 0ull};
+        if constexpr (LANES > 1) {
+            d = dk[0];
+#pragma unroll
+            for (int k = 0; k + 1 < AHEAD; ++k) dk[k] = dk[k + 1];
+        } else {
+            const int tn = start(q);
 #pragma unroll 2
-        for (int r = t + p; r < tn; r += LANES) {
-            BoxSum in = v[(r + a.n) * gj], out = v[r * gj];
-            sar128(in.lo, in.hi, eb - (int)in.e);
-            sar128(out.lo, out.hi, eb - (int)out.e);
-            add128(dl, dh, in.lo, in.hi);
-            sub128(dl, dh, out.lo, out.hi);
-            dc += in.cnt - out.cnt;
+            for (int r = t; r < tn; ++r) slide(d, v[(r + a.n) * gj], v[r * gj]);
+            t = tn;
         }
-        col_reduce<LANES>(dl, dh, dc);
-        add128(lo, hi, dl, dh);
-        cnt += dc;
-        t = tn;
+        col_reduce<LANES>(d.lo, d.hi, d.cnt);
+        add128(lo, hi, d.lo, d.hi);
+        cnt += d.cnt;
     }
 }
 
@@ -410,30 +478,35 @@ __device__ __forceinline__ void box_cols(const BoxArgs& a, const int vb) {
     float* __restrict__ o = reinterpret_cast<float*>(a.means + m) + img;
     const size_t gj = (size_t)a.gj;
     const int q0 = a.q0 + run * RUN, q1 = min(q0 + RUN, a.q1);
+    auto start = [&](int q) { return box_start(a.xo + q * a.gs, a.nx, a.nsize); };
+    int emax = 1, emin = 0x7fffffff;
+    exp_range<LANES>(ve, gj, start(q0) + p, start(q1 - 1) + a.n, emax, emin);
     if constexpr (LANES == 1) {
         // a long run whose rows' units lie far apart goes in pieces of kColRun,
         // so that its small boxes keep the unit a short run gives them
-        const int t0 = box_start(a.xo + q0 * a.gs, a.nx, a.nsize);
-        const int t1 = box_start(a.xo + (q1 - 1) * a.gs, a.nx, a.nsize) + a.n;
-        int emax = 1, emin = 0x7fffffff;
-#pragma unroll 4
-        for (int r = t0; r < t1; ++r) {
-            const int e = __ldg(ve + r * gj);
-            emax = max(emax, e);
-            emin = min(emin, e);
+        if (emax - emin > 8) {
+            for (int q = q0; q < q1; q += kColRun) {
+                const int qe = min(q + kColRun, q1);
+                int e1 = 1;
+                exp_range<1>(ve, gj, start(q), start(qe - 1) + a.n, e1, emin);
+                box_run<1>(a, v, o, gj, q, qe, p, act, e1);
+            }
+            return;
         }
-        const int piece = emax - emin > 8 ? kColRun : RUN;
-        for (int q = q0; q < q1; q += piece) box_run<1>(a, v, ve, o, gj, q, min(q + piece, q1), p, act);
     } else {
-        box_run<LANES>(a, v, ve, o, gj, q0, q1, p, act);
+#pragma unroll
+        for (int k = 1; k < LANES; k <<= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, k, LANES));
     }
+    box_run<LANES>(a, v, o, gj, q0, q1, p, act, emax);
 }
 
 __device__ __forceinline__ void k_box_cols_body(const BoxArgs& a, const int vb, const int) {
     grid_dep_wait();  // the row sums come from the kernel before
     box_cols<kColLanes>(a, vb);
 }
-FLCT_MULTI_KERNEL(__launch_bounds__(128), k_box_cols, BoxArgs)
+// 7 blocks an SM: without the cap (93 registers) 512^2 -s 1 takes 50 us of
+// prepass instead of 46, and 1024^2 -s 4 38 instead of 36
+FLCT_MULTI_KERNEL(__launch_bounds__(128, 7), k_box_cols, BoxArgs)
 
 __device__ __forceinline__ void k_box_cols_long_body(const BoxArgs& a, const int vb, const int) {
     grid_dep_wait();

@@ -34,16 +34,19 @@ constexpr int kBoxWarps = 4;
 constexpr int kRowSpan = 544;
 // Column pass: runs of grid rows, starting at multiples of their length (the
 // units of a run's box sums depend on the rows it reads).  Small grids want
-// short chains: four lanes share a run of four.  From kColLong grid points
-// (both frames) on there are lanes enough, and a lane of its own per run of 16
-// reads each row sum (n + 15) / 16 times instead of (n + 3) / 4.  Prepass of
-// 2048^2 -s 2 at box 64 265 -> 187 us, 769 x 1023 every pixel at box 48 152 ->
-// 80, 1500 x 1800 at box 12 317 -> 163; at 524,288 points (512^2 every pixel,
-// box 32) 46 against 45, at 131,072 (1024^2 -s 4) 36 against 75.  Two kernels,
-// as one with both branches costs the small grids 0.5-1 us of code.
+// short chains: four lanes share a run of four.  From kColLong (gs + 1) / 2
+// grid points (both frames) on there are lanes enough, and a lane of its own
+// per run of 16 reads each row sum (n + 15 gs) / 16 gs times instead of
+// (n + 3 gs) / 4 gs.  Prepass, short against long runs: every pixel at box 32,
+// 300 x 310 26 against 33 us, 400^2 35 / 35, 512^2 46 / 38; at box 64 400^2
+// 44 / 42, 450 x 455 61 / 47; -s 2: 700^2 at box 24 40 / 49, 1000 x 900 63 / 62
+// (82 / 71 at box 64), 2048^2 at box 64 265 / 172; -s 3: 1500^2 at box 40
+// 103 / 110; 769 x 1023 every pixel at box 48 152 / 75, 1500 x 1800 at box 12
+// 317 / 157.  Two kernels, as one with both branches costs the small grids
+// 0.5-1 us of code.
 constexpr int kColRun = 4, kColLanes = 4;
 constexpr int kColRunLong = 16;
-constexpr long kColLong = 800000;
+constexpr long kColLong = 320000;
 
 // Local means for the boxes the grid needs, from exact box sums
 // (fixsum.cuh).  Grid point (q, m) is pixel (xo + q gs, yo + m gs) (gs = 1,
