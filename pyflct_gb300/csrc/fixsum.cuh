@@ -11,9 +11,11 @@
 // span's largest.  Row sums carry their span's exponent; a run of box sums
 // down a grid column takes the largest exponent of the row sums it reads
 // and shifts the others down to it (again dropping only bits 2^62 below the
-// largest).  Spans and runs are fixed by the frame geometry alone, and
-// integer sums are exact, so every box sum is the same for any order, run
-// length or band split, and is rounded once when it becomes a double.
+// largest); boxes above 64 x 64 take a unit two bits higher, so that their up
+// to 2^14 values stay below 2^127 too.  Spans and runs are fixed by the frame
+// geometry alone, and integer sums are exact, so every box sum is the same
+// for any order, run length or band split, and is rounded once when it
+// becomes a double.
 // Non-finite inputs are counted instead (NaN, +inf and -inf in 16-bit
 // fields) and give the value a sequential double sum would have: NaN with
 // any NaN or with both infinities, else the infinity present.

@@ -479,6 +479,8 @@ __device__ __forceinline__ void box_cols(const BoxArgs& a, const int vb) {
     const size_t gj = (size_t)a.gj;
     const int q0 = a.q0 + run * RUN, q1 = min(q0 + RUN, a.q1);
     auto start = [&](int q) { return box_start(a.xo + q * a.gs, a.nx, a.nsize); };
+    // boxes above 64 x 64 hold up to 2^14 values: two more bits of headroom
+    const int room = a.n > 64 ? 2 : 0;
     int emax = 1, emin = 0x7fffffff;
     exp_range<LANES>(ve, gj, start(q0) + p, start(q1 - 1) + a.n, emax, emin);
     if constexpr (LANES == 1) {
@@ -489,7 +491,7 @@ __device__ __forceinline__ void box_cols(const BoxArgs& a, const int vb) {
                 const int qe = min(q + kColRun, q1);
                 int e1 = 1;
                 exp_range<1>(ve, gj, start(q), start(qe - 1) + a.n, e1, emin);
-                box_run<1>(a, v, o, gj, q, qe, p, act, e1);
+                box_run<1>(a, v, o, gj, q, qe, p, act, e1 + room);
             }
             return;
         }
@@ -497,7 +499,7 @@ __device__ __forceinline__ void box_cols(const BoxArgs& a, const int vb) {
 #pragma unroll
         for (int k = 1; k < LANES; k <<= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, k, LANES));
     }
-    box_run<LANES>(a, v, o, gj, q0, q1, p, act, emax);
+    box_run<LANES>(a, v, o, gj, q0, q1, p, act, emax + room);
 }
 
 __device__ __forceinline__ void k_box_cols_body(const BoxArgs& a, const int vb, const int) {
