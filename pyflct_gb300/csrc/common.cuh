@@ -142,16 +142,30 @@ __device__ __forceinline__ void publish_counters(const unsigned* src, unsigned* 
     }
 }
 
-// Exact float -> double with integer operations for normal floats and
+// Division of 0 <= n < 2^31 by a fixed d >= 1: the high word of n times
+// floor(2^32 / d) + 1 is the quotient or one more.
+struct FastDiv {
+    int d = 1;
+    unsigned m = 0;
+    FastDiv() = default;
+    __host__ __device__ explicit FastDiv(int div) : d(div), m(div > 1 ? 0xffffffffu / (unsigned)div + 1u : 0u) {}
+    __device__ __forceinline__ int div(int n) const {
+        if (d == 1) return n;
+        const int q = (int)__umulhi((unsigned)n, m);
+        return q - ((unsigned)q * (unsigned)d > (unsigned)n ? 1 : 0);
+    }
+};
+
+// f 2^K as a double, exact, with integer operations for normal floats and
 // zeros; subnormals, infinities and NaN take the conversion instruction.
+template <int K = 0>
 __device__ __forceinline__ double f2d(float f) {
-    const unsigned u = __float_as_uint(f);
-    const unsigned E = (u >> 23) & 0xffu;
-    const unsigned long long s = (unsigned long long)(u >> 31) << 63;
-    if (E == 0u && (u & 0x7fffffu) == 0u) return __longlong_as_double((long long)s);
-    if (E == 0u || E == 255u) return f2d_slow(f);
-    return __longlong_as_double(
-        (long long)(s | ((unsigned long long)(E + 896u) << 52) | ((unsigned long long)(u & 0x7fffffu) << 29)));
+    const unsigned u = __float_as_uint(f), m = u & 0x7fffffffu, s = u & 0x80000000u;
+    if (m - 0x00800000u < 0x7f000000u)
+        return __hiloint2double((int)(((m >> 3) + 0x38000000u + ((unsigned)K << 20)) | s), (int)(u << 29));
+    if (m == 0u) return __hiloint2double((int)s, 0);
+    const double d = f2d_slow(f);
+    return K == 0 ? d : __dmul_rn(d, K < 0 ? 1.0 / (1 << (K < 0 ? -K : 0)) : (double)(1 << (K > 0 ? K : 0)));
 }
 
 // Power-of-two factor bringing a non-negative float (given as its bits) into

@@ -909,6 +909,8 @@ InterpArgs interp_args(const Job& j, const JobBufs& b, int i0, int i1, Pub pub) 
     ia.nx = j.nx;
     ia.ny = j.ny;
     ia.skip = j.d.skip;
+    ia.skd = FastDiv(std::max(1, j.d.skip));
+    ia.ntc = FastDiv((j.ny + kTileC - 1) / kTileC);
     ia.xoff = j.d.xoff;
     ia.yoff = j.d.yoff;
     ia.gx = j.d.icnt;

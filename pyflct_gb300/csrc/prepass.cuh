@@ -72,6 +72,7 @@ constexpr int kTileR = 32, kTileC = 32, kInterpThreads = 256;
 // The velocity pipeline's skip-grid interpolation (FP32 arithmetic).
 struct InterpArgs {
     int nx, ny, skip, xoff, yoff;
+    FastDiv skd, ntc;         // divisions by skip and by the tiles per tile row
     int gx, gy;               // grid counts along the slow / fast axis
     const float2* grid;       // (vx, vy) per grid point [gx][gy]
     double *vx, *vy, *vm;

@@ -45,20 +45,6 @@ __host__ __device__ __forceinline__ int meta_I(unsigned m) { return (int)(m & 0x
 __host__ __device__ __forceinline__ int meta_J(unsigned m) { return (int)((m >> 15) & 0x7fffu); }
 __host__ __device__ __forceinline__ bool meta_flag(unsigned m) { return (m >> 30) & 1u; }
 
-// Division of 0 <= n < 2^31 by a fixed d >= 1: the high word of n times
-// floor(2^32 / d) + 1 is the quotient or one more.
-struct FastDiv {
-    int d = 1;
-    unsigned m = 0;
-    FastDiv() = default;
-    __host__ __device__ explicit FastDiv(int div) : d(div), m(div > 1 ? 0xffffffffu / (unsigned)div + 1u : 0u) {}
-    __device__ __forceinline__ int div(int n) const {
-        if (d == 1) return n;
-        const int q = (int)__umulhi((unsigned)n, m);
-        return q - ((unsigned)q * (unsigned)d > (unsigned)n ? 1 : 0);
-    }
-};
-
 // Where the window of pixel (i, j) finds its local means: one float4
 // (f1 hi, f2 hi, f1 lo, f2 lo) per grid point [gi][gj], grid point (q, m) =
 // pixel (xo + q gs, yo + m gs).
