@@ -157,9 +157,9 @@ __device__ __forceinline__ void k_fit_hires_body(const FitArgs& a, const int vb,
             const int ixx = mi / NI, iyy = mi - (mi / NI) * NI;
             double ssx = 0., ssy = 0.;
             if (ixx > 0 && ixx < NI - 1 && iyy > 0 && iyy < NI - 1) {
-                double v[9];
+                float v[9];
 #pragma unroll
-                for (int k = 0; k < 9; ++k) v[k] = f2d(s_pk[warp][(ixx - 1 + k / 3) * NI + (iyy - 1 + k % 3)]);
+                for (int k = 0; k < 9; ++k) v[k] = s_pk[warp][(ixx - 1 + k / 3) * NI + (iyy - 1 + k % 3)];
                 fit3x3(v, &ssx, &ssy);
                 // times rangex / (nxinterp - 1) = 2 / 20 (flct.c:1625-1628)
                 ssx = dm(ssx, 2.) / 20.;
