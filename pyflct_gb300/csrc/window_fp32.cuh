@@ -57,13 +57,28 @@ struct WinArgs {
 };
 
 // Launch shape of the box-N kernel.  Variant V = 0 is the default; V = 1
-// is the autotuner's alternative: twice the teams per CTA where that CTA
-// still fits twice per SM in shared memory and has at most 512 threads,
-// else half the teams, with no register cap.  A window's arithmetic is the
-// same in both; only the windows per CTA and the occupancy differ.
+// is the autotuner's alternative: of a base of 8, 4 or 2 teams twice as many
+// where that CTA still fits twice per SM in shared memory and has at most 512
+// threads, else half (box 52: two), with no register cap.  A window's
+// arithmetic is the same in both; only the windows per CTA and the occupancy
+// differ.
+template <int N>
+constexpr int win_teams_base() {
+    return (N <= 8) ? (128 / N) : (N <= 20 || N == 32) ? 8 : (N <= 44) ? 4 : 2;
+}
+// The default is the base except where a sweep of 1..16 teams found better:
+// few teams wait less for one another at the CTA's barriers, many share the
+// code they fetch, and either should fill its last warp and the SM's warp
+// slots.  us per 65,536 windows, base -> here: box 20 91 -> 85, 28 180 -> 170,
+// 36 360 -> 331, 40 381 -> 356, 52 886 -> 760 (one CTA of 364 threads an SM),
+// 60 1007 -> 979.  No better than the base: 12, 24, 44, 48, and 64, where six
+// teams take 921 us for 929 but 15.14 ms for 15.06 a 2048^2 -s 2 call.
 template <int N>
 constexpr int win_teams0() {
-    return (N <= 8) ? (128 / N) : (N <= 20 || N == 32) ? 8 : (N <= 44) ? 4 : 2;
+    return N == 52                        ? 7
+           : N == 20 || N == 36 || N == 40 ? 3
+           : N == 28 || N == 60           ? 1
+                                          : win_teams_base<N>();
 }
 // Boxes 16 and 32 (whole-warp teams) read rows and row weights 16 bytes at a
 // time and look for the peak's place only after its value: 8% fewer
@@ -87,7 +102,8 @@ constexpr size_t win_smem(int teams) {
 }
 template <int N>
 constexpr int win_teams_alt() {
-    constexpr int t = win_teams0<N>();
+    constexpr int t = win_teams_base<N>();
+    if (N == 52) return 2;
     return (2 * t * N <= 512 && 2 * win_smem<N>(2 * t) <= 227 * 1024) ? 2 * t : (t > 1 ? t / 2 : 1);
 }
 
