@@ -31,11 +31,20 @@ __global__ void __launch_bounds__(256) k_copy_arrays(CopyArgs a) {
     }
 }
 
+// The kernel moves doubles: every array has to start on their boundary (a view
+// into a file's bytes may not), which the runtime's copies do not ask for.
+bool kernel_copies(const double* const* src, double* const* dst, int count, size_t n) {
+    if (count > 3 || n * sizeof(double) > kHostKernelBytes) return false;
+    uintptr_t any = 0;
+    for (int k = 0; k < count; ++k) any |= reinterpret_cast<uintptr_t>(src[k]) | reinterpret_cast<uintptr_t>(dst[k]);
+    return any % alignof(double) == 0;
+}
+
 }  // namespace
 
 cudaError_t copy_arrays(const double* const* src, double* const* dst, int count, size_t n, cudaMemcpyKind kind,
                         bool direct, cudaStream_t st) {
-    if (direct && count <= 3 && n * sizeof(double) <= kHostKernelBytes) {
+    if (direct && kernel_copies(src, dst, count, n)) {
         CopyArgs a{};
         for (int k = 0; k < count; ++k) {
             a.src[k] = src[k];

@@ -1,0 +1,77 @@
+"""Which route a host array takes: a kernel that loads and stores its doubles
+in place, or the runtime's copies.  On the stand-in runtime, without a GPU."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import _fake_cuda
+from pyflct_gb300.flct import make_params
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    h = _fake_cuda.Host(_fake_cuda.load(tmp_path_factory.mktemp("fake")))
+    yield h
+    h.close()
+
+
+N = 40
+
+
+def at(off):
+    """N x N doubles, `off` bytes past a 16-byte boundary."""
+    b = np.zeros(N * N * 8 + 32, np.uint8)
+    a = (-b.ctypes.data) % 16 + off
+    return b[a:a + N * N * 8].view(np.float64).reshape(N, N)
+
+
+def ptr(a):
+    return C.cast(a.ctypes.data, C.POINTER(C.c_double))
+
+
+def routes(log):
+    """(arrays copied by the kernel in, out), (by the runtime in, out)."""
+    kern = [int(x.split()[3]) for x in log if "k_copy_arrays" in x]
+    whole = [x.split() for x in log if x.startswith("copy ") and x.split()[2] == str(N * N * 8)]
+    return kern, [sum(x[1] == k for x in whole) for k in "12"]
+
+
+CALLS = {"velocity": (2, 3), "shift": (1, 1), "warp": (3, 1)}
+
+
+def call(host, name, arrays):
+    p = make_params(1.0, 1.0, 3.0)
+    if name == "velocity":
+        return host.call("velocity", C.byref(p), ptr(arrays[0]), ptr(arrays[1]), N, N, *[ptr(a) for a in arrays[2:]])
+    if name == "shift":
+        return host.call("shift_frac2d", ptr(arrays[0]), C.c_double(0.5), C.c_double(0.25), ptr(arrays[1]), N, N, 1)
+    return host.call("warp_frac2d", *[ptr(a) for a in arrays], N, N, 1)
+
+
+@pytest.mark.parametrize("name", CALLS)
+def test_aligned_arrays_take_the_kernel(host, name):
+    nin, nout = CALLS[name]
+    for off in (0, 8):
+        rc, log = call(host, name, [at(off) for _ in range(nin + nout)])
+        assert rc == 0 and routes(log) == ([nin, nout], [0, 0])
+
+
+@pytest.mark.parametrize("name", CALLS)
+@pytest.mark.parametrize("off", [1, 2, 4, 12])
+def test_unaligned_arrays_take_the_runtimes_copies(host, name, off):
+    nin, nout = CALLS[name]
+    for k in range(nin + nout):
+        arrays = [at(off if q == k else 0) for q in range(nin + nout)]
+        assert arrays[k].ctypes.data % 8
+        rc, log = call(host, name, arrays)
+        assert rc == 0
+        # the side of the call that holds the array, all of it
+        assert routes(log) == (([nout], [nin, 0]) if k < nin else ([nin], [0, nout])), k
+
+
+def test_numpy_hands_unaligned_arrays_through():
+    """Why the check is the library's: a view 4 bytes into a buffer is C-contiguous float64."""
+    from pyflct_gb300.flct import _f64
+    a = np.frombuffer(bytearray(8 * 100 + 4), np.float64, count=100, offset=4).reshape(10, 10)
+    assert _f64(a).ctypes.data % 8 == a.ctypes.data % 8
