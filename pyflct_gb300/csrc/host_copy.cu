@@ -32,11 +32,18 @@ __global__ void __launch_bounds__(256) k_copy_arrays(CopyArgs a) {
 }
 
 // The kernel moves doubles: every array has to start on their boundary (a view
-// into a file's bytes may not), which the runtime's copies do not ask for.
+// into a file's bytes may not), which the runtime's copies do not ask for.  It
+// also moves all arrays at once: results that share memory, where a later one
+// is to stay, are left to copies one after another.
 bool kernel_copies(const double* const* src, double* const* dst, int count, size_t n) {
     if (count > 3 || n * sizeof(double) > kHostKernelBytes) return false;
     uintptr_t any = 0;
     for (int k = 0; k < count; ++k) any |= reinterpret_cast<uintptr_t>(src[k]) | reinterpret_cast<uintptr_t>(dst[k]);
+    for (int k = 1; k < count; ++k)
+        for (int q = 0; q < k; ++q) {
+            const uintptr_t a = reinterpret_cast<uintptr_t>(dst[k]), b = reinterpret_cast<uintptr_t>(dst[q]);
+            if ((a < b ? b - a : a - b) < n * sizeof(double)) return false;
+        }
     return any % alignof(double) == 0;
 }
 

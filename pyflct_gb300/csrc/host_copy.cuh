@@ -12,7 +12,8 @@ namespace flct {
 // copies of about 10 us of latency each.  A call on 201 x 101 frames 147 ->
 // 105 us, 512^2 -s 3i 225 -> 178, 1024^2 -s 4i 532 -> 490.  Larger arrays
 // gain nothing by it, and pages that were never touched cost a kernel more
-// than the copy engine.  Arrays off an 8-byte boundary go to the runtime.
+// than the copy engine.  Arrays off an 8-byte boundary, and results that share
+// memory, go to the runtime.
 constexpr size_t kHostKernelBytes = 1u << 24;
 
 // `count` arrays of n doubles, src[k] to dst[k], ordered on st.  direct: the

@@ -75,3 +75,20 @@ def test_numpy_hands_unaligned_arrays_through():
     from pyflct_gb300.flct import _f64
     a = np.frombuffer(bytearray(8 * 100 + 4), np.float64, count=100, offset=4).reshape(10, 10)
     assert _f64(a).ctypes.data % 8 == a.ctypes.data % 8
+
+
+def test_outputs_that_share_memory_are_written_in_order(host):
+    """One scratch array for two results holds the later one, as copies one after another leave it."""
+    f, g, a, b = (at(0) for _ in range(4))
+    c = np.zeros(N * N + N)  # and two that overlap in part
+    p = make_params(1.0, 1.0, 3.0)
+    for out in ((a, a, b), (a, b, a), (b, a, a), (c[:N * N], a, c[N:])):
+        rc, log = host.call("velocity", C.byref(p), ptr(f), ptr(g), N, N, *[ptr(o) for o in out])
+        assert rc == 0 and routes(log) == ([2], [0, 3])
+        assert [int(x.split()[3], 16) for x in log if x.startswith("copy 2 %d " % (N * N * 8))] == [o.ctypes.data for o in out]
+    # neighbours do not
+    rc, log = host.call("velocity", C.byref(p), ptr(f), ptr(f), N, N, ptr(c[:N * N]), ptr(a), ptr(b))
+    assert rc == 0 and routes(log) == ([2, 3], [0, 0])
+    whole = np.zeros((3, N, N))
+    rc, log = host.call("velocity", C.byref(p), ptr(f), ptr(g), N, N, *[ptr(o) for o in whole])
+    assert rc == 0 and routes(log) == ([2, 3], [0, 0])
