@@ -1808,6 +1808,16 @@ flct_status enqueue_banded(flct_ctx* ctx, const Job& j, const Bands& bd, int for
     return FLCT_OK;
 }
 
+// A host-buffer call's copy kernels use the caller's arrays until they are
+// done: whichever way the call returns before its own wait, it waits here.
+struct CallerArrays {
+    cudaStream_t st;
+    bool in_use = true;
+    ~CallerArrays() {
+        if (in_use) cudaStreamSynchronize(st);
+    }
+};
+
 bool page_locked(const void* p) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
@@ -2325,6 +2335,7 @@ flct_status flct_gpu_velocity(flct_ctx* ctx, const flct_params* p, const double*
         }
     }
     CK(cudaEventRecord(ctx->ev[4], st));
+    CallerArrays arrays{st};
     {
         const double* src[] = {f1, f2};
         double* dst[] = {(double*)ctx->b_f1.p, (double*)ctx->b_f2.p};
@@ -2334,10 +2345,7 @@ flct_status flct_gpu_velocity(flct_ctx* ctx, const flct_params* p, const double*
     flct_status s = flct_gpu_velocity_device(ctx, p, (const double*)ctx->b_f1.p, (const double*)ctx->b_f2.p,
                                              nx, ny, (double*)ctx->b_vx.p, (double*)ctx->b_vy.p,
                                              (double*)ctx->b_vm.p, st);
-    if (s != FLCT_OK) {
-        cudaStreamSynchronize(st);
-        return s;
-    }
+    if (s != FLCT_OK) return s;
     {
         const double* src[] = {(const double*)ctx->b_vx.p, (const double*)ctx->b_vy.p, (const double*)ctx->b_vm.p};
         double* dst[] = {vx, vy, vm};
@@ -2347,6 +2355,7 @@ flct_status flct_gpu_velocity(flct_ctx* ctx, const flct_params* p, const double*
     }
     CK(cudaEventRecord(ctx->ev[6], st));
     CK(cudaStreamSynchronize(st));
+    arrays.in_use = false;
     s = collect_timing(ctx);
     ctx->timing.ms_h2d = ev_ms(ctx->ev[4], ctx->ev[5]);
     ctx->timing.ms_d2h = ev_ms(ctx->ev[3], ctx->ev[6]);
@@ -2544,6 +2553,7 @@ flct_status flct_gpu_shift_frac2d(flct_ctx* ctx, const double* arr, double delx,
     // warp.c:811-820: shifts normalised by the axis lengths; transp swaps them
     const double dxarg = transp ? -dely / ((double)nx) : -delx / ((double)nx);
     const double dyarg = transp ? -delx / ((double)ny) : -dely / ((double)ny);
+    CallerArrays arrays{st};
     {
         double* dst = (double*)ctx->b_f1.p;
         CK(copy_arrays(&arr, &dst, 1, n, cudaMemcpyHostToDevice, ctx->host_direct, st));
@@ -2572,6 +2582,7 @@ flct_status flct_gpu_shift_frac2d(flct_ctx* ctx, const double* arr, double delx,
         CK(copy_arrays(&src, &out, 1, n, cudaMemcpyDeviceToHost, ctx->host_direct, st));
     }
     CK(cudaStreamSynchronize(st));
+    arrays.in_use = false;
     ctx->timing = flct_timing{};
     ctx->timing.launches = fft ? 5 + (ls.p[0].chirp || ls.p[1].chirp) : 7;
     ctx->timing.ms_total = ev_ms(ctx->ev[0], ctx->ev[1]);
@@ -2599,6 +2610,15 @@ flct_status flct_gpu_warp_frac2d(flct_ctx* ctx, const double* arr, const double*
     ENSURE(ctx->b_aux1, fft ? line_setup_bytes(ls) : (size_t)(nx + ny) * sizeof(float2) + 64);
     float2* twx = (float2*)ctx->b_aux1.p;
     float2* twy = twx + nx;
+    // the spectral sum: tensor cores (split FP16, half spectrum) unless
+    // FLCT_WARP_SUM=fp32 asks for the FP32 CUDA-core kernel
+    const char* form = getenv("FLCT_WARP_SUM");
+    const bool tc = !(form && strcmp(form, "fp32") == 0);
+    if (tc) {
+        ENSURE(ctx->b_whs, warp_tc_split_bytes(nx, ny, ctx->nsm));
+        ENSURE(ctx->b_wmisc, warp_tc_misc_bytes(ctx->nsm));
+    }
+    CallerArrays arrays{st};
     {
         const double* src[] = {arr, delx, dely};
         double* dst[] = {(double*)ctx->b_f1.p, (double*)ctx->b_f2.p, (double*)ctx->b_vy.p};
@@ -2619,14 +2639,8 @@ flct_status flct_gpu_warp_frac2d(flct_ctx* ctx, const double* arr, const double*
     CK(launch_warp_phase((const double*)ctx->b_f2.p, (const double*)ctx->b_vy.p, nx, ny, transp,
                          (float4*)ctx->b_means.p, st));
     CK(cudaEventRecord(ctx->ev[1], st));
-    // the spectral sum: tensor cores (split FP16, half spectrum) unless
-    // FLCT_WARP_SUM=fp32 asks for the FP32 CUDA-core kernel
-    const char* form = getenv("FLCT_WARP_SUM");
-    const bool tc = !(form && strcmp(form, "fp32") == 0);
     unsigned wstatus = 0;
     if (tc) {
-        ENSURE(ctx->b_whs, warp_tc_split_bytes(nx, ny, ctx->nsm));
-        ENSURE(ctx->b_wmisc, warp_tc_misc_bytes(ctx->nsm));
         unsigned long long stall_ns = 0;  // test hook: see k_wt_sum
         if (const char* w = getenv("FLCT_TEST_WARP_STALL_NS")) stall_ns = strtoull(w, nullptr, 10);
         CK(launch_warp_sum_tc((const float2*)ctx->b_s2.p, (const float4*)ctx->b_means.p, nx, ny, ctx->b_whs.p,
@@ -2643,6 +2657,7 @@ flct_status flct_gpu_warp_frac2d(flct_ctx* ctx, const double* arr, const double*
     }
     if (tc) CK(cudaMemcpyAsync(&wstatus, (unsigned*)ctx->b_wmisc.p + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    arrays.in_use = false;
     ctx->timing = flct_timing{};
     ctx->timing.launches = (fft ? 5 + (ls.p[0].chirp || ls.p[1].chirp) : 4) + 1 + (tc ? 3 : 1);
     ctx->timing.ms_prepass = ev_ms(ctx->ev[0], ctx->ev[1]);
