@@ -235,8 +235,14 @@ cudaError_t launch_lines2(const LineArgs2& a, int axes, int nsm, cudaStream_t st
         pts = std::max(pts, line_pts(x.p));
     }
     void (*kern)(LineArgs2) = pts == 16 ? k_lines<16, 1024> : threads > 256 ? k_lines<8, 1024> : k_lines<8, 256>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
+    // the limit is the kernel's, shared by every context and thread: always
+    // what its longest line takes (256 threads carry 2048 points: 17 KB)
+    if (pts == 16 || threads > 256) {
+        const int most = pts == 16 ? kLineMax : 8192;
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)((most + most / 16) * sizeof(float2)));
+        if (e != cudaSuccess) return e;
+    }
     return launch_kernel(kern, dim3(std::min(groups, nsm * 16), axes), dim3(threads), smem, st, true, a);
 }
 

@@ -317,14 +317,18 @@ __global__ void __launch_bounds__(256) k_warp_sum(const float2* __restrict__ F, 
 
 // ------------------------------------------------------------ host ----
 
+// The axis kernels' limit of dynamic shared memory: the kernel's, shared by
+// every context and thread, so always what the longest axis takes.
+constexpr int kAxisSmem = kWarpMaxAxis * (int)sizeof(float2);
+
 cudaError_t launch_axis_fast(int mode, bool real_in, const void* in, int nrows, int L, const float2* tab,
                              float2* out, cudaStream_t st) {
     dim3 g((L + 63) / 64, (nrows + 15) / 16);
     const size_t sm = (size_t)L * sizeof(float2);
     cudaError_t e = cudaSuccess;
-#define FLCT_AF(M, R)                                                                                \
-    e = cudaFuncSetAttribute(k_axis_fast<M, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
-    if (e != cudaSuccess) return e;                                                                  \
+#define FLCT_AF(M, R)                                                                                    \
+    e = cudaFuncSetAttribute(k_axis_fast<M, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAxisSmem); \
+    if (e != cudaSuccess) return e;                                                                      \
     k_axis_fast<M, R><<<g, 256, sm, st>>>(in, nrows, L, tab, out);
     if (mode == 0 && real_in) { FLCT_AF(0, true) }
     else if (mode == 0) { FLCT_AF(0, false) }
@@ -340,11 +344,11 @@ cudaError_t launch_axis_slow(int mode, const float2* in, int ncols, int L, const
     const size_t sm = (size_t)L * sizeof(float2);
     cudaError_t e;
     if (mode == 0) {
-        e = cudaFuncSetAttribute(k_axis_slow<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        e = cudaFuncSetAttribute(k_axis_slow<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAxisSmem);
         if (e != cudaSuccess) return e;
         k_axis_slow<0><<<g, 256, sm, st>>>(in, ncols, L, tab, out);
     } else {
-        e = cudaFuncSetAttribute(k_axis_slow<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        e = cudaFuncSetAttribute(k_axis_slow<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAxisSmem);
         if (e != cudaSuccess) return e;
         k_axis_slow<1><<<g, 256, sm, st>>>(in, ncols, L, tab, out);
     }
