@@ -59,9 +59,9 @@ struct WinArgs {
 // Launch shape of the box-N kernel.  Variant V = 0 is the default; V = 1
 // is the autotuner's alternative: of a base of 8, 4 or 2 teams twice as many
 // where that CTA still fits twice per SM in shared memory and has at most 512
-// threads, else half (box 52: two), with no register cap.  A window's
-// arithmetic is the same in both; only the windows per CTA and the occupancy
-// differ.
+// threads, else half (boxes 52 and 60, whose default is not the base: the
+// base's two), with no register cap.  A window's arithmetic is the same in
+// both; only the windows per CTA and the occupancy differ.
 template <int N>
 constexpr int win_teams_base() {
     return (N <= 8) ? (128 / N) : (N <= 20 || N == 32) ? 8 : (N <= 44) ? 4 : 2;
@@ -103,13 +103,14 @@ constexpr size_t win_smem(int teams) {
 template <int N>
 constexpr int win_teams_alt() {
     constexpr int t = win_teams_base<N>();
-    if (N == 52) return 2;
+    if (N == 52 || N == 60) return 2;
     return (2 * t * N <= 512 && 2 * win_smem<N>(2 * t) <= 227 * 1024) ? 2 * t : (t > 1 ? t / 2 : 1);
 }
 
 template <int N, int V = 0>
 struct WinShape {
     static constexpr int TEAMS = V == 0 ? win_teams0<N>() : win_teams_alt<N>();
+    static_assert(win_teams_alt<N>() != win_teams0<N>(), "the tuner would time one shape twice");
     static constexpr int THREADS = N * TEAMS;
     static constexpr int LD = win_ld<N>();   // row stride, float2
     static constexpr int BUF = N * LD;       // float2 per team
