@@ -472,15 +472,18 @@ void tune_save(flct_ctx* ctx) {
     fprintf(f, "{\"device\": \"%s\", \"entries\": [\n", ctx->device_name.c_str());
     size_t k = 0;
     for (const auto& e : ctx->tune) {
-        fprintf(f, "  {\"box\": %d, \"form\": %d, \"grid_div\": %d, \"ns_per_window\": %.4f, \"variant\": %d}%s\n",
-                e.first, e.second.form, e.second.grid_div, e.second.ns_per_window, e.second.variant,
-                (++k < ctx->tune.size()) ? "," : "");
+        fprintf(f, "  {\"box\": %d, \"form\": %d, \"grid_div\": %d, \"ns_per_window\": %.4f, \"variant\": %d",
+                e.first, e.second.form, e.second.grid_div, e.second.ns_per_window, e.second.variant);
+        // the launch shapes it was measured with
+        if (const WinEntry* we = find_win(e.first)) fprintf(f, ", \"teams\": [%d, %d]", we->teams[0], we->teams[1]);
+        fprintf(f, "}%s\n", (++k < ctx->tune.size()) ? "," : "");
     }
     fprintf(f, "]}\n");
     fclose(f);
 }
 
-// Reads entries written by tune_save (one per line) for this device name.
+// Reads entries written by tune_save (one per line) for this device name,
+// but for those measured with other launch shapes than this library's.
 void tune_load(flct_ctx* ctx) {
     if (ctx->tune_path.empty()) return;
     FILE* f = fopen(ctx->tune_path.c_str(), "r");
@@ -504,6 +507,12 @@ void tune_load(flct_ctx* ctx) {
             int v = 0;
             const char* qv = strstr(q, "\"variant\"");
             if (qv && sscanf(qv, "\"variant\": %d", &v) == 1 && (v == 0 || v == 1)) t.variant = v;
+            const WinEntry* we = find_win(box);
+            const char* qt = strstr(q, "\"teams\"");
+            int t0 = 0, t1 = 0;
+            if (we && qt &&
+                (sscanf(qt, "\"teams\": [%d, %d]", &t0, &t1) != 2 || t0 != we->teams[0] || t1 != we->teams[1]))
+                continue;
             ctx->tune[box] = t;
         }
     }
