@@ -187,38 +187,42 @@ __global__ void __launch_bounds__(128) k_line_setup(LineSetup a) {
 
 constexpr int kRadices[] = {16, 15, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
 
-// Fewest passes for n: exhaustive over descending radices (lengths have few divisors).
-bool split(int n, int from, int depth, int* cur, int& best, int* out) {
-    if (n == 1) {
-        if (depth < best) {
-            best = depth;
-            for (int k = 0; k < depth; ++k) out[k] = cur[k];
+// The lengths up to kLineMax without a prime factor above 13 and the fewest
+// passes of each, made once per process (20 us): a search at every call took
+// 24 us for a length of many divisors and up to 1.1 ms for a chirp's length,
+// more than its transforms.
+struct Lengths {
+    unsigned char passes[kLineMax + 1] = {};  // 0: a larger prime factor
+    unsigned short smooth[1024];              // ascending
+    int count = 0;
+    Lengths() {
+        for (int m = 1; m <= kLineMax; ++m) {
+            if (m > 1 && !passes[m]) continue;
+            if (count < 1024) smooth[count++] = (unsigned short)m;
+            for (int r : kRadices)
+                if (m * r <= kLineMax && (!passes[m * r] || passes[m * r] > passes[m] + 1))
+                    passes[m * r] = (unsigned char)(passes[m] + 1);
         }
-        return true;
+        passes[1] = 1;
     }
-    if (depth + 1 >= best || depth == 8) return false;
-    bool ok = false;
-    for (int k = from; k < (int)(sizeof(kRadices) / sizeof(int)); ++k)
-        if (n % kRadices[k] == 0) {
-            cur[depth] = kRadices[k];
-            ok |= split(n / kRadices[k], k, depth + 1, cur, best, out);
-        }
-    return ok;
+};
+const Lengths& lengths() {
+    static const Lengths t;
+    return t;
 }
 
-// Passes of a length-n transform (0: n has a prime factor above 13), their
-// radices a byte each.
-int passes_of(int n, unsigned long long* radices) {
-    int cur[9], out[9], best = 9;
-    if (radices) *radices = 0;
-    if (n == 1) return 1;
-    int rest = n;
-    for (int f : {2, 3, 5, 7, 11, 13})
-        while (rest % f == 0) rest /= f;
-    if (rest > 1) return 0;
-    if (!split(n, 0, 0, cur, best, out)) return 0;
-    for (int k = best - 1; k >= 0 && radices; --k) *radices = *radices << 8 | (unsigned)out[k];
-    return best;
+// The radices of a length's fewest passes, a byte each, the largest first.
+unsigned long long radices_of(int n) {
+    const Lengths& t = lengths();
+    unsigned long long out = 0;
+    for (int shift = 0; n > 1; shift += 8)
+        for (int r : kRadices)
+            if (n % r == 0 && (n == r ? 0 : t.passes[n / r]) == t.passes[n] - 1) {
+                out |= (unsigned long long)r << shift;
+                n /= r;
+                break;
+            }
+    return out;
 }
 
 // Points a thread carries through a pass: 8 while a line's threads fit a CTA.
@@ -252,25 +256,27 @@ LinePlan line_plan(int L, int chirp_min) {
     LinePlan p;
     p.L = L;
     if (L < 1) return p;
-    if (L <= kLineMax && (p.npass = passes_of(L, &p.radices))) {
+    const Lengths& t = lengths();
+    if (L <= kLineMax && t.passes[L]) {
         p.M = L;
-    } else if (L < chirp_min) {
+    } else if (L < chirp_min || 2 * (long)L - 1 > kLineMax) {
         return p;
     } else {
-        // chirp length: the smooth one of least work
+        // chirp length: the smooth one of least work, up to the next power of two
         long best = -1;
-        for (int m = 2 * L - 1; m <= kLineMax && m <= 4 * L; ++m) {
-            const int n = passes_of(m, nullptr);
-            if (n && (best < 0 || (long)m * (n + 1) < best)) {
-                best = (long)m * (n + 1);
-                p.M = m;
+        for (const unsigned short* m = std::lower_bound(t.smooth, t.smooth + t.count, 2 * L - 1);
+             m < t.smooth + t.count; ++m) {
+            const long work = (long)*m * (t.passes[*m] + 1);
+            if (best < 0 || work < best) {
+                best = work;
+                p.M = *m;
             }
-            if ((m & (m - 1)) == 0 && best > 0) break;
+            if ((*m & (*m - 1)) == 0) break;
         }
-        if (best < 0) return p;
-        p.npass = passes_of(p.M, &p.radices);
         p.chirp = true;
     }
+    p.npass = t.passes[p.M];
+    p.radices = radices_of(p.M);
     p.T = (p.M + line_pts(p) - 1) / line_pts(p);
     return p;
 }
