@@ -1641,9 +1641,10 @@ struct Bands {
 bool plan_bands(const flct_ctx* ctx, const Job& j, Bands* bd) {
     if (j.d.global || j.d.rel_thresh || j.gi < 1) return false;
     const int run = col_run(j);
-    for (int nb = std::min(ctx->host_bands_max, j.gi / (2 * run)); nb >= 2; --nb) {
+    for (int nb = std::min(ctx->host_bands_max, j.gi / (2 * kColRun)); nb >= 2; --nb) {
         bool ok = true;
-        // band starts at multiples of the column pass's run
+        // band starts at multiples of the column pass's run (a band without a
+        // run is refused below)
         for (int b = 0; b <= nb; ++b)
             bd->Q[b] = (b == nb) ? j.gi : (int)((long)j.gi * b / nb) / run * run;
         for (int b = 0; b <= nb; ++b) bd->R[b] = (b == 0) ? 0 : (b == nb) ? j.nx : j.xo + bd->Q[b] * j.gs;

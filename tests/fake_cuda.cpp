@@ -16,6 +16,7 @@ std::string g_log;
 std::map<const void*, std::string> g_kernels;
 long g_calls = 0, g_fail_at = 0;
 bool g_failed = false;
+bool g_pinned = false;  // what host pointers are said to be
 int g_int = 0;  // what a 4-byte copy from the device returns, if not 0
 dim3 g_grid, g_block;
 size_t g_smem = 0;
@@ -60,6 +61,7 @@ void fake_reset(long fail_at) {
 }
 int fake_failed() { return g_failed; }
 void fake_int(int v) { g_int = v; }
+void fake_pinned(int v) { g_pinned = v; }
 
 void** __cudaRegisterFatBinary(void*) {
     static void* h;
@@ -172,7 +174,7 @@ cudaError_t cudaHostGetDevicePointer(void** d, void* h, unsigned) {
 }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
     memset(a, 0, sizeof(*a));
-    a->type = cudaMemoryTypeUnregistered;
+    a->type = g_pinned ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
     return cudaSuccess;
 }
 static cudaError_t copy(const char* what, void* d, const void* s, size_t n, cudaMemcpyKind k) {
