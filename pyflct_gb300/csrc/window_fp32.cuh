@@ -60,7 +60,7 @@ struct WinArgs {
 // is the autotuner's alternative: of a base of 8, 4 or 2 teams twice as many
 // where that CTA still fits twice per SM in shared memory and has at most 512
 // threads, else half (boxes 52 and 60, whose default is not the base: the
-// base's two), with no register cap.  A window's arithmetic is the same in
+// base's two; box 16: four, for the bands of host calls), with no register cap.  A window's arithmetic is the same in
 // both; only the windows per CTA and the occupancy differ.
 template <int N>
 constexpr int win_teams_base() {
@@ -86,25 +86,29 @@ constexpr int win_teams0() {
 // cache (29 KB of code; at 32 KB it asked the cache behind for 57% of its
 // bandwidth).  65,536 windows: box 16 44.7 -> 42.7 us, box 32 165.6 -> 159.4.
 // Boxes 4 and 8 gain nothing by it (9.9 -> 11.9, 17.7 -> 18.0), and teams that
-// share warps pay more for the peak's second look than they save.
-template <int N>
-constexpr bool win_quads() { return N == 16 || N == 32; }
+// share warps pay more for the peak's second look than they save.  Shape 1,
+// which bands of host calls launch with one set of windows per CTA, keeps the
+// plain loop: it has less to set up (page-locked calls, with quads -> without:
+// 1024^2 at box 32 3,119 -> 3,028 us, 100 x 2500 at box 16 281 -> 270).
+template <int N, int V>
+constexpr bool win_quads() { return V == 0 && (N == 16 || N == 32); }
 // 16-byte row reads want a stride of n + 2 to stay on distinct banks, 8-byte
 // ones n + 1; the row weights are four shifted copies, read from any start.
-template <int N>
-constexpr int win_ld() { return win_quads<N>() ? N + 2 : N + 1; }
-template <int N>
-constexpr size_t win_weights() { return win_quads<N>() ? (size_t)4 * (N / 2 + 1) * 16 : 0; }
-template <int N>
+template <int N, int V>
+constexpr int win_ld() { return win_quads<N, V>() ? N + 2 : N + 1; }
+template <int N, int V>
+constexpr size_t win_weights() { return win_quads<N, V>() ? (size_t)4 * (N / 2 + 1) * 16 : 0; }
+template <int N, int V>
 constexpr size_t win_smem(int teams) {
-    return 32 * teams + win_weights<N>() + ((3 * N + 1) * 4 + 15) / 16 * 16 + (size_t)N * 8 +
-           (size_t)teams * N * win_ld<N>() * 8;
+    return 32 * teams + win_weights<N, V>() + ((3 * N + 1) * 4 + 15) / 16 * 16 + (size_t)N * 8 +
+           (size_t)teams * N * win_ld<N, V>() * 8;
 }
 template <int N>
 constexpr int win_teams_alt() {
     constexpr int t = win_teams_base<N>();
     if (N == 52 || N == 60) return 2;
-    return (2 * t * N <= 512 && 2 * win_smem<N>(2 * t) <= 227 * 1024) ? 2 * t : (t > 1 ? t / 2 : 1);
+    if (N == 16) return 4;
+    return (2 * t * N <= 512 && 2 * win_smem<N, 1>(2 * t) <= 227 * 1024) ? 2 * t : (t > 1 ? t / 2 : 1);
 }
 
 template <int N, int V = 0>
@@ -112,13 +116,13 @@ struct WinShape {
     static constexpr int TEAMS = V == 0 ? win_teams0<N>() : win_teams_alt<N>();
     static_assert(win_teams_alt<N>() != win_teams0<N>(), "the tuner would time one shape twice");
     static constexpr int THREADS = N * TEAMS;
-    static constexpr int LD = win_ld<N>();   // row stride, float2
+    static constexpr int LD = win_ld<N, V>();  // row stride, float2
     static constexpr int BUF = N * LD;       // float2 per team
-    static constexpr size_t g_off = 32 * TEAMS + win_weights<N>();
+    static constexpr size_t g_off = 32 * TEAMS + win_weights<N, V>();
     static constexpr size_t tw_off = g_off + ((3 * N + 1) * 4 + 15) / 16 * 16;
     static constexpr size_t head = tw_off + (size_t)N * 8;
     static constexpr size_t smem = head + (size_t)TEAMS * BUF * 8;  // |c| reuses the buffer
-    static_assert(smem == win_smem<N>(TEAMS), "shared-memory layout");
+    static_assert(smem == win_smem<N, V>(TEAMS), "shared-memory layout");
     // CTAs per SM the register allocation is held to (0: no constraint).
     // Box 32: 2 CTAs of 8 teams at 128 registers (159.5 us for 65,536 windows;
     // 161.4 at 20 warps per SM, 190 at 12).  Box 16: 7 CTAs of 4 warps (46.8
@@ -154,7 +158,7 @@ k_window_fp32(WinArgs a) {
     // shuffles; other team widths share warps and go through shared memory
     // and the CTA barrier.
     constexpr bool kWarp = (32 % N == 0);
-    constexpr bool kQuads = win_quads<N>();
+    constexpr bool kQuads = win_quads<N, V>();
     const unsigned tmask =
         (N == 32) ? 0xffffffffu : (((1u << (N & 31)) - 1u) << ((threadIdx.x & 31) & ~(unsigned)(N - 1)));
     auto team_sync = [] {

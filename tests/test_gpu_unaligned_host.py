@@ -31,8 +31,8 @@ def test_inputs_and_outputs(off):
     from pyflct_gb300 import _lib, synth
     from pyflct_gb300.flct import flct, make_params, shift_frac2d, warp_frac2d
     rng = np.random.default_rng(off)
-    f1 = synth.kfield((61, 53), rng)
-    f2 = synth.fourier_shift(f1, 0.4, -0.3)
+    f1 = np.ascontiguousarray(synth.kfield((61, 53), rng))
+    f2 = np.ascontiguousarray(synth.fourier_shift(f1, 0.4, -0.3))
     d = synth.smooth_shift(f1.shape, rng, rms=1.0)
     ctx = _lib.context(0)
     want = flct(f1, f2, 1.0, 1.0, 3.0)

@@ -40,3 +40,22 @@ def test_bands_of_few_rows(host, shape, sigma, run, bands):
     assert len(out) == bands
     assert [o for o, _ in out] == list(np.cumsum([0] + [n for _, n in out]))[:-1] and sum(n for _, n in out) == nx
     assert all(o % run == 0 for o, _ in out)
+
+
+@pytest.mark.parametrize("sigma, n", [(4.0, 16), (8.0, 32)])
+def test_bands_launch_the_light_shape(host, sigma, n):
+    """One set of windows per CTA: few of them, and none of the tables that pay over many sets."""
+    shape = (200, 250)
+    a = [np.zeros(shape) for _ in range(5)]
+    p = [x.ctypes.data_as(C.POINTER(C.c_double)) for x in a]
+    host.lib.fake_pinned(1)
+    try:
+        rc, log = host.call("velocity", C.byref(make_params(1.0, 1.0, sigma)), p[0], p[1], *shape, *p[2:])
+    finally:
+        host.lib.fake_pinned(0)
+    assert rc == 0
+    wins = [x.split() for x in log if x.startswith("launch") and "k_window_fp32ILi%d" % n in x]
+    assert len(wins) == 5
+    for x in wins:
+        teams = int(x[5]) // n
+        assert teams == 4 and int(x[-1]) < teams * n * (n + 2) * 8  # rows n + 1 apart, no copies of the weights
