@@ -90,28 +90,30 @@ __global__ void k_gz(const double* __restrict__ f1, const double* __restrict__ f
     }
 }
 
-// Tile of a direct DFT: 32 LP lines by 16 KQ frequencies, LP pairs of lines
-// by KQ frequencies per thread, on packed FMAs (two lines an instruction).
+// Tile of a direct DFT: 2 TL LP lines by 256 / TL KQ frequencies, LP pairs of
+// lines by KQ frequencies per thread, on packed FMAs (two lines an instruction).
 // Every output adds its L terms from j = 0 up, the real part x.x w.x after
 // -x.y w.y, so results do not depend on the tile.  Chunks of kDftChunk points
 // of the lines and their twiddles tw[(j k) mod L] go through shared memory;
-// a thread steps the index of its twiddle column.  Bound by the FP32 pipe (65% busy; 4 FMAs per point and output, 2
-// where only the real part is wanted).  The four passes of a 1000 x 1200
-// call: 5.1 -> 0.83 ms against one output a thread, which read the table once
-// per 4 FMAs.
+// a thread steps the index of its twiddle column.  Bound by the FP32 pipe (65%
+// busy; 4 FMAs per point and output, 2 where only the real part is wanted).
+// The four passes of a 1000 x 1200 call: 5.1 -> 0.83 ms against one output a
+// thread, which read the table once per 4 FMAs.  Tiles of 8 lines for as few:
+// 8 x 10007 3.31 -> 1.29 ms, 8 x 4096 0.42 -> 0.37; no gain below (8 x 1000
+// 0.113 -> 0.127).
 constexpr int kDftChunk = 16;
 
-template <int DIR, int LP, int KQ, bool REAL_OUT>
+template <int DIR, int TL, int LP, int KQ, bool REAL_OUT>
 __global__ void __launch_bounds__(256) k_dft_rows(const float2* __restrict__ in, float2* __restrict__ out, int L,
                                                   int lines, const float2* __restrict__ tw,
                                                   const unsigned* __restrict__ scale) {
-    constexpr int J = kDftChunk, WL = 32 * LP, WK = 16 * KQ;
+    constexpr int J = kDftChunk, TK = 256 / TL, WL = 2 * TL * LP, WK = TK * KQ;
     __shared__ __align__(16) float xr[J][WL + 2], xi[J][WL + 2];
     __shared__ float2 ws[J][WK];
     grid_dep_wait();
-    // a thread's outputs lie 16 frequencies (32 lines) apart, so that a warp
+    // a thread's outputs lie TK frequencies (2 TL lines) apart, so that a warp
     // reads whole rows of ws
-    const int t = threadIdx.x, tk = t & 15, tl = 2 * (t >> 4);
+    const int t = threadIdx.x, tk = t % TK, tl = 2 * (t / TK);
     const int k0 = blockIdx.x * WK, l0 = blockIdx.y * WL;
     const float c1 = scale ? pow2_scale(scale[0]) : 1.f, c2 = scale ? pow2_scale(scale[1]) : 1.f;
     // this thread's twiddle column, from its row on
@@ -122,7 +124,7 @@ __global__ void __launch_bounds__(256) k_dft_rows(const float2* __restrict__ in,
     float2 ax[LP][KQ] = {}, ay[LP][KQ] = {};
     // the next chunk travels while this one is summed; half a warp reads 16
     // points of a line
-    constexpr int NX = WL * J / 256, NW = J / WR;
+    constexpr int NX = (WL * J + 255) / 256, NW = J / WR;
     const int jx = t % J, lx = t / J;
     float2 nx[NX], nw[NW];
     auto fetch = [&](int j0) {
@@ -143,6 +145,7 @@ __global__ void __launch_bounds__(256) k_dft_rows(const float2* __restrict__ in,
         __syncthreads();
 #pragma unroll
         for (int q = 0; q < NX; ++q) {
+            if (WL * J < 256 && lx >= WL) break;
             xr[jx][lx + q * (256 / J)] = nx[q].x * c1;
             xi[jx][lx + q * (256 / J)] = nx[q].y * c2;
         }
@@ -159,12 +162,12 @@ __global__ void __launch_bounds__(256) k_dft_rows(const float2* __restrict__ in,
             float2 w[KQ];
 #pragma unroll
             for (int p = 0; p < LP; ++p) {
-                re[p] = *reinterpret_cast<const float2*>(&xr[j][tl + 32 * p]);
-                im[p] = *reinterpret_cast<const float2*>(&xi[j][tl + 32 * p]);
+                re[p] = *reinterpret_cast<const float2*>(&xr[j][tl + 2 * TL * p]);
+                im[p] = *reinterpret_cast<const float2*>(&xi[j][tl + 2 * TL * p]);
                 ni[p] = make_float2(-im[p].x, -im[p].y);
             }
 #pragma unroll
-            for (int q = 0; q < KQ; ++q) w[q] = ws[j][tk + 16 * q];
+            for (int q = 0; q < KQ; ++q) w[q] = ws[j][tk + TK * q];
 #pragma unroll
             for (int p = 0; p < LP; ++p)
 #pragma unroll
@@ -179,22 +182,73 @@ __global__ void __launch_bounds__(256) k_dft_rows(const float2* __restrict__ in,
     for (int p = 0; p < LP; ++p)
 #pragma unroll
         for (int q = 0; q < KQ; ++q) {
-            const int l = l0 + tl + 32 * p, kk = k0 + tk + 16 * q;
+            const int l = l0 + tl + 2 * TL * p, kk = k0 + tk + TK * q;
             if (kk >= L) continue;
             if (l < lines) out[(size_t)l * L + kk] = make_float2(ax[p][q].x, ay[p][q].x);
             if (l + 1 < lines) out[(size_t)(l + 1) * L + kk] = make_float2(ax[p][q].y, ay[p][q].y);
         }
 }
 
+// The same sums, one output a thread, for one to three lines so long that tiles
+// of 64 frequencies would share SMs: there the twiddle reads bound both, and
+// these keep more of them in flight.  1 x 10007 (whole call) 1.26 -> 0.91 ms,
+// 3 x 10007 1.27 -> 0.91, 1 x 30000 10.6 -> 6.7; 2 x 30000, two rounds of
+// blocks, would take 14.0 for the tiles' 10.6.
+template <int DIR, bool REAL_OUT>
+__global__ void __launch_bounds__(256) k_dft_long(const float2* __restrict__ in, float2* __restrict__ out, int L,
+                                                  const float2* __restrict__ tw, const unsigned* __restrict__ scale) {
+    constexpr int J = 2048;
+    __shared__ float2 x[J];
+    grid_dep_wait();
+    const int k = blockIdx.x * 256 + threadIdx.x;
+    const float2* const src = in + (size_t)blockIdx.y * L;
+    const float c1 = scale ? pow2_scale(scale[0]) : 1.f, c2 = scale ? pow2_scale(scale[1]) : 1.f;
+    float ax = 0.f, ay = 0.f;
+    int idx = 0;  // (j k) mod L
+    for (int j0 = 0; j0 < L; j0 += J) {
+        const int jn = min(J, L - j0);
+        __syncthreads();
+        for (int j = threadIdx.x; j < jn; j += 256) {
+            const float2 v = src[j0 + j];
+            x[j] = make_float2(v.x * c1, v.y * c2);
+        }
+        __syncthreads();
+        if (k >= L) continue;
+        for (int j = 0; j < jn; ++j) {
+            float2 w = __ldg(tw + idx);
+            if (DIR > 0) w.y = -w.y;
+            const float2 v = x[j];
+            ax = fmaf(v.x, w.x, fmaf(-v.y, w.y, ax));
+            if (!REAL_OUT) ay = fmaf(v.x, w.y, fmaf(v.y, w.x, ay));
+            idx += k;
+            if (idx >= L) idx -= L;
+        }
+    }
+    if (k < L) out[(size_t)blockIdx.y * L + k] = make_float2(ax, ay);
+}
+
 cudaError_t launch_dft_rows(bool inverse, bool real_out, const float2* in, float2* out, int L, int lines,
                             const float2* tw, const unsigned* scale, int nsm, cudaStream_t st) {
-    // the widest tile that still gives every SM one
+    // the widest tile that still gives every SM one, but none that is mostly
+    // lines that are not there: up to 32 lines 32 x 32, up to 8 lines 8 x 64
+    // once tiles of 32 x 16 would share SMs
     auto grid = [&](int wl, int wk) { return dim3((L + wk - 1) / wk, (lines + wl - 1) / wl); };
     auto tiles = [&](int wl, int wk) { return (long)grid(wl, wk).x * grid(wl, wk).y; };
-    const bool wide = tiles(64, 64) >= nsm, mid = tiles(32, 32) >= nsm;
-#define FLCT_DFT(D, LP, KQ, R) \
-    launch_kernel(k_dft_rows<D, LP, KQ, R>, grid(32 * LP, 16 * KQ), dim3(256), 0, st, true, in, out, L, lines, tw, scale)
-#define FLCT_DFT_TILE(D, R) (wide ? FLCT_DFT(D, 2, 4, R) : mid ? FLCT_DFT(D, 1, 2, R) : FLCT_DFT(D, 1, 1, R))
+    const bool few = lines <= 8 && tiles(32, 16) > nsm;
+    const dim3 one((L + 255) / 256, lines);  // one output a thread: in one round of the SMs
+    if (few && tiles(8, 64) > nsm && (long)one.x * one.y <= nsm) {
+        auto* kern = !inverse ? k_dft_long<-1, false> : real_out ? k_dft_long<1, true> : k_dft_long<1, false>;
+        return launch_kernel(kern, one, dim3(256), 0, st, true, in, out, L, tw, scale);
+    }
+    const bool wide = lines > 32 && tiles(64, 64) >= nsm, mid = tiles(32, 32) >= nsm;
+#define FLCT_DFT(D, TL, LP, KQ, R)                                                                             \
+    launch_kernel(k_dft_rows<D, TL, LP, KQ, R>, grid(2 * TL * LP, 256 / TL * KQ), dim3(256), 0, st, true, in, \
+                  out, L, lines, tw, scale)
+#define FLCT_DFT_TILE(D, R)             \
+    (few    ? FLCT_DFT(D, 4, 1, 1, R)   \
+     : wide ? FLCT_DFT(D, 16, 2, 4, R)  \
+     : mid  ? FLCT_DFT(D, 16, 1, 2, R)  \
+            : FLCT_DFT(D, 16, 1, 1, R))
     return !inverse ? FLCT_DFT_TILE(-1, false) : real_out ? FLCT_DFT_TILE(1, true) : FLCT_DFT_TILE(1, false);
 #undef FLCT_DFT_TILE
 #undef FLCT_DFT
