@@ -2576,22 +2576,44 @@ flct_status flct_gpu_shift_frac2d(flct_ctx* ctx, const double* arr, double delx,
         ls.darg[1] = dyarg;
         ls.ph[0] = (double2*)ctx->b_aux2.p;
         ls.ph[1] = ls.ph[0] + nx;
-        CK(launch_shift_fft((const double*)ctx->b_f1.p, ls, (float2*)ctx->b_s1.p, (float2*)ctx->b_s2.p,
-                            (double*)ctx->b_vx.p, ctx->nsm, st));
-    } else {
-        CK(launch_shift_vector(nx, dxarg, (double2*)ctx->b_aux2.p, sx, st));
-        CK(launch_shift_vector(ny, dyarg, (double2*)ctx->b_aux2.p, sy, st));
-        CK(launch_axis_fast(0, true, ctx->b_f1.p, nx, ny, sy, (float2*)ctx->b_s1.p, st));
-        CK(launch_axis_slow(0, (const float2*)ctx->b_s1.p, ny, nx, sx, (float2*)ctx->b_s2.p, st));
-        CK(launch_real_part((const float2*)ctx->b_s2.p, (long)n, (double*)ctx->b_vx.p, st));
     }
-    CK(cudaEventRecord(ctx->ev[1], st));
-    populate_output(out, n * sizeof(double));
-    {
+    volatile unsigned* const odd = (unsigned*)ctx->hctr + 2;
+    auto results = [&](int ex) -> flct_status {  // of the image times 2^-ex, times 2^ex
+        *odd = 0u;
+        if (fft) {
+            CK(launch_shift_fft((const double*)ctx->b_f1.p, ls, (float2*)ctx->b_s1.p, (float2*)ctx->b_s2.p,
+                                (double*)ctx->b_vx.p, ctx->hctr_dev + 2, ctx->nsm, st));
+        } else {
+            CK(launch_shift_vector(nx, dxarg, (double2*)ctx->b_aux2.p, sx, st));
+            CK(launch_shift_vector(ny, dyarg, (double2*)ctx->b_aux2.p, sy, st));
+            CK(launch_axis_fast(0, true, ctx->b_f1.p, nx, ny, sy, (float2*)ctx->b_s1.p, st));
+            CK(launch_axis_slow(0, (const float2*)ctx->b_s1.p, ny, nx, sx, (float2*)ctx->b_s2.p, st));
+            CK(launch_real_part((const float2*)ctx->b_s2.p, (long)n, (double*)ctx->b_vx.p, st));
+        }
+        if (ex) CK(launch_scale((double*)ctx->b_vx.p, (long)n, std::ldexp(1.0, ex), st));
+        CK(cudaEventRecord(ctx->ev[1], st));
+        populate_output(out, n * sizeof(double));
         const double* src = (const double*)ctx->b_vx.p;
         CK(copy_arrays(&src, &out, 1, n, cudaMemcpyDeviceToHost, ctx->host_direct, st));
+        CK(cudaStreamSynchronize(st));
+        return FLCT_OK;
+    };
+    s = results(0);
+    if (s != FLCT_OK) return s;
+    if (*odd) {
+        double mx = 0.0;
+        ENSURE(ctx->b_wmisc, 64);
+        CK(cudaMemsetAsync(ctx->b_wmisc.p, 0, sizeof(double), st));
+        CK(launch_abs_max((const double*)ctx->b_f1.p, (long)n, (unsigned long long*)ctx->b_wmisc.p, st));
+        CK(cudaMemcpyAsync(&mx, ctx->b_wmisc.p, sizeof(double), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        if (std::isfinite(mx) && mx > 0.0 && (mx < kShiftLo || mx > kShiftHi)) {
+            const int ex = std::max(-1000, std::min(1000, std::ilogb(mx)));
+            CK(launch_scale((double*)ctx->b_f1.p, (long)n, std::ldexp(1.0, -ex), st));
+            s = results(ex);
+            if (s != FLCT_OK) return s;
+        }
     }
-    CK(cudaStreamSynchronize(st));
     arrays.in_use = false;
     ctx->timing = flct_timing{};
     ctx->timing.launches = fft ? 5 + (ls.p[0].chirp || ls.p[1].chirp) : 7;

@@ -200,17 +200,42 @@ __global__ void __launch_bounds__(256) k_transpose_c(const float2* __restrict__ 
         if (c0 + i < cols && r0 + threadIdx.x < rows) out[(size_t)(c0 + i) * rows + r0 + threadIdx.x] = t[threadIdx.x][i];
 }
 
-// out[c][r] = Re(in[r][c]) as double, 32 x 32 tiles.
+// out[c][r] = Re(in[r][c]) as double, 32 x 32 tiles.  *odd (mapped host memory)
+// is set where a warp's values are not finite or none reaches kShiftLo.
 __global__ void __launch_bounds__(256) k_transpose_re(const float2* __restrict__ in, int rows, int cols,
-                                                      double* __restrict__ out) {
+                                                      double* __restrict__ out, unsigned* odd) {
     __shared__ float t[32][33];
     grid_dep_wait();
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+    unsigned mx = 0u;
     for (int i = threadIdx.y; i < 32; i += 8)
-        if (r0 + i < rows && c0 + threadIdx.x < cols) t[i][threadIdx.x] = in[(size_t)(r0 + i) * cols + c0 + threadIdx.x].x;
+        if (r0 + i < rows && c0 + threadIdx.x < cols) {
+            const float v = in[(size_t)(r0 + i) * cols + c0 + threadIdx.x].x;
+            t[i][threadIdx.x] = v;
+            mx = max(mx, __float_as_uint(v) & 0x7fffffffu);
+        }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    const bool rows_here = r0 + (int)threadIdx.y < rows;
+    if (rows_here && (mx >= 0x7f800000u || __uint_as_float(mx) < (float)kShiftLo) && threadIdx.x == 0) {
+        *(volatile unsigned*)odd = 1u;
+        __threadfence_system();
+    }
     __syncthreads();
     for (int i = threadIdx.y; i < 32; i += 8)
         if (c0 + i < cols && r0 + threadIdx.x < rows) out[(size_t)(c0 + i) * rows + r0 + threadIdx.x] = (double)t[threadIdx.x][i];
+}
+
+__global__ void k_scale(double* __restrict__ x, long n, double f) {
+    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) x[k] *= f;
+}
+
+// The bits of max |x[k]| (a NaN's above all others).
+__global__ void k_abs_max(const double* __restrict__ x, long n, unsigned long long* __restrict__ mx) {
+    unsigned long long m = 0ull;
+    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x)
+        m = max(m, (unsigned long long)__double_as_longlong(x[k]) & ~(1ull << 63));
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(mx, m);
 }
 
 __global__ void k_real_part(const float2* __restrict__ in, long n, double* __restrict__ out) {
@@ -361,8 +386,18 @@ cudaError_t launch_shift_vector(int n, double darg, double2* scratch, float2* v,
     return cudaGetLastError();
 }
 
-cudaError_t launch_shift_fft(const double* in, const LineSetup& s, float2* buf1, float2* buf2, double* out, int nsm,
-                             cudaStream_t st) {
+cudaError_t launch_scale(double* x, long n, double f, cudaStream_t st) {
+    k_scale<<<(int)std::min<long>((n + 255) / 256, 4096), 256, 0, st>>>(x, n, f);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_abs_max(const double* x, long n, unsigned long long* mx, cudaStream_t st) {
+    k_abs_max<<<(int)std::min<long>((n + 255) / 256, 4096), 256, 0, st>>>(x, n, mx);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_shift_fft(const double* in, const LineSetup& s, float2* buf1, float2* buf2, double* out, unsigned* odd,
+                             int nsm, cudaStream_t st) {
     const int nx = s.p[0].L, ny = s.p[1].L;
     cudaError_t e = launch_line_setup(s, st);
     // fast axis: rows of the image, then the slow axis as rows of the transpose
@@ -373,7 +408,7 @@ cudaError_t launch_shift_fft(const double* in, const LineSetup& s, float2* buf1,
     if (e == cudaSuccess) e = launch_lines(kLineShift, s.p[0], s.t[0], buf2, false, buf1, ny, s.ph[0], nsm, st);
     if (e == cudaSuccess)
         e = launch_kernel(k_transpose_re, dim3((nx + 31) / 32, (ny + 31) / 32), dim3(32, 8), 0, st, true, buf1, ny, nx,
-                          out);
+                          out, odd);
     return e;
 }
 

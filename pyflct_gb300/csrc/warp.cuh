@@ -18,9 +18,19 @@ cudaError_t launch_axis_slow(int mode, const float2* in, int ncols, int L, const
 cudaError_t launch_shift_vector(int n, double darg, double2* scratch, float2* v, cudaStream_t st);
 cudaError_t launch_twiddles(int L, int sign, float2* tw, cudaStream_t st);
 // shift_frac2d by transforms (axis 0 slow, 1 fast, both with line plans and
-// phase factors): buf1 / buf2 nx * ny float2 each; out nx * ny doubles on the device
-cudaError_t launch_shift_fft(const double* in, const LineSetup& s, float2* buf1, float2* buf2, double* out, int nsm,
-                             cudaStream_t st);
+// phase factors): buf1 / buf2 nx * ny float2 each; out nx * ny doubles on the
+// device; *odd (mapped host memory, 0 before) is set where results are not
+// finite or very small.  Transforms and convolution grow values by up to 2^28
+// where circulant sums stay at the image's size, so an image whose largest
+// value lies outside [kShiftLo, kShiftHi] leaves FP32's range on the way: it
+// goes through once more, scaled by a power of two.
+constexpr double kShiftLo = 0x1p-60, kShiftHi = 0x1p+96;
+cudaError_t launch_shift_fft(const double* in, const LineSetup& s, float2* buf1, float2* buf2, double* out, unsigned* odd,
+                             int nsm, cudaStream_t st);
+// x[k] *= f, k < n
+cudaError_t launch_scale(double* x, long n, double f, cudaStream_t st);
+// *mx (0 before) = the bits of max |x[k]|, a NaN's above all others
+cudaError_t launch_abs_max(const double* x, long n, unsigned long long* mx, cudaStream_t st);
 // F = forward 2-D DFT of a real nx x ny image by transforms: buf1 nx * ny
 // float2 scratch, F nx * ny float2 (natural [ii][jj] order)
 cudaError_t launch_dft2_fft(const double* in, const LineSetup& s, float2* buf1, float2* F, int nsm, cudaStream_t st);
