@@ -2637,7 +2637,10 @@ flct_status flct_gpu_warp_frac2d(flct_ctx* ctx, const double* arr, const double*
     ENSURE(ctx->b_s1, n * sizeof(float2));
     ENSURE(ctx->b_s2, n * sizeof(float2));
     ENSURE(ctx->b_means, n * sizeof(float4));
-    LineSetup ls = line_setup(nx, ny, 1);
+    // small images with a rough axis: the DFT matrices are fewer launches
+    // (whole call, with convolutions -> without: 3 x 37 94 -> 88 us, 17 x 17 99
+    // -> 91; 37 x 37 106 either way, 41 x 41 107 -> 111, 64 x 17 96 -> 117)
+    LineSetup ls = line_setup(nx, ny, std::max(nx, ny) <= 37 ? 64 : 1);
     const bool fft = ls.p[0].npass && ls.p[1].npass;
     ENSURE(ctx->b_aux1, fft ? line_setup_bytes(ls) : (size_t)(nx + ny) * sizeof(float2) + 64);
     float2* twx = (float2*)ctx->b_aux1.p;

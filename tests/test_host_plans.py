@@ -36,3 +36,12 @@ def quickest(host, name, nx, ny):
 def test_rough_lengths_cost_the_host_no_more(host, name, n):
     smooth = quickest(host, name, 3, 5120)  # a longer line without a convolution
     assert quickest(host, name, 3, n) <= smooth + 60e-6
+
+
+@pytest.mark.parametrize("shape, lines", [((3, 37), False), ((17, 17), False), ((2, 17), False), ((37, 37), False),
+                                          ((16, 36), True), ((3, 41), True), ((64, 17), True), ((17, 200), True)])
+def test_small_warps_of_rough_sides_skip_the_convolutions(host, shape, lines):
+    a = [np.zeros(shape) for _ in range(4)]
+    rc, log = host.call("warp_frac2d", *[x.ctypes.data_as(C.POINTER(C.c_double)) for x in a], *shape, 1)
+    assert rc == 0
+    assert any("k_lines" in x for x in log) == lines and any("k_axis_fast" in x for x in log) != lines
