@@ -51,7 +51,8 @@ bool kernel_copies(const double* const* src, double* const* dst, int count, size
 
 cudaError_t copy_arrays(const double* const* src, double* const* dst, int count, size_t n, cudaMemcpyKind kind,
                         bool direct, cudaStream_t st) {
-    if (direct && kernel_copies(src, dst, count, n)) {
+    const bool staged = kind == cudaMemcpyHostToDevice && count * n * sizeof(double) <= kHostStagedBytes;
+    if (direct && !staged && kernel_copies(src, dst, count, n)) {
         CopyArgs a{};
         for (int k = 0; k < count; ++k) {
             a.src[k] = src[k];

@@ -15,6 +15,11 @@ namespace flct {
 // than the copy engine.  Arrays off an 8-byte boundary, and results that share
 // memory, go to the runtime.
 constexpr size_t kHostKernelBytes = 1u << 24;
+// Copies in of up to this many bytes in all are taken by the runtime as they
+// are enqueued, while a kernel would first have to fetch them: 2-3 us of a
+// 60 us call (shift of 17 x 17 63.6 -> 60.4 us, velocity of 24 x 24 66.3 ->
+// 63.6); three arrays of 18 KB gain nothing.
+constexpr size_t kHostStagedBytes = 1u << 15;
 
 // `count` arrays of n doubles, src[k] to dst[k], ordered on st.  direct: the
 // GPU may use pageable host addresses (cudaDevAttrPageableMemoryAccess with

@@ -16,7 +16,7 @@ def host(tmp_path_factory):
     h.close()
 
 
-N = 40
+N = 72
 
 
 def at(off):
@@ -92,3 +92,14 @@ def test_outputs_that_share_memory_are_written_in_order(host):
     whole = np.zeros((3, N, N))
     rc, log = host.call("velocity", C.byref(p), ptr(f), ptr(g), N, N, *[ptr(o) for o in whole])
     assert rc == 0 and routes(log) == ([2, 3], [0, 0])
+
+
+@pytest.mark.parametrize("n, kernel", [(4, False), (32, False), (45, False), (46, True), (64, True)])
+def test_small_copies_in_are_the_runtimes(host, n, kernel):
+    """Up to 32 KB of inputs in all; results go by the kernel."""
+    a = [np.zeros((n, n)) for _ in range(5)]
+    rc, log = host.call("velocity", C.byref(make_params(1.0, 1.0, 0.0)), *[ptr(x) for x in a[:2]], n, n, *[ptr(x) for x in a[2:]])
+    assert rc == 0
+    copies = [x.split() for x in log if x.startswith("copy 1 ") and x.split()[2] == str(8 * n * n)]
+    assert len(copies) == (0 if kernel else 2)
+    assert [int(x.split()[3]) for x in log if "k_copy_arrays" in x] == ([2, 3] if kernel else [3])

@@ -17,7 +17,7 @@ def lib(tmp_path_factory):
     return _fake_cuda.load(tmp_path_factory.mktemp("fake"))
 
 
-N = 48
+N = 72
 A = [np.zeros((N, N)) for _ in range(5)]
 P = [a.ctypes.data_as(C.POINTER(C.c_double)) for a in A]
 PAR = {"velocity": make_params(1.0, 1.0, 3.0), "interpolated": make_params(1.0, 1.0, 3.0, thresh="0.1", skip="3i"),
