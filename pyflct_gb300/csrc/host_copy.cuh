@@ -29,7 +29,11 @@ cudaError_t copy_arrays(const double* const* src, double* const* dst, int count,
 
 // Makes a caller's output pages present while the GPU computes: 8 MB of fresh
 // pages cost a copy 377 us through GPU faults, 52 us once they are there.
-// Leaves the contents as they are; errors are of no consequence.
-void populate_output(void* p, size_t bytes);
+// Leaves the contents as they are.  False where the host may not write them (or
+// the system cannot tell): a copy kernel must not either, a store to such a page
+// is a fault of the device where the runtime's copy returns an error.  (Results
+// of less than a page are touched: without permission that is the host's own
+// fault, as a copy by the host would be.)
+bool populate_output(void* p, size_t bytes);
 
 }  // namespace flct

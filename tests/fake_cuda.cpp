@@ -3,6 +3,8 @@
 // once, kernels do not run, and every call is written to a log.  A chosen
 // call can be made to fail.
 #include <cuda_runtime_api.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <cstdio>
 #include <cstdlib>
@@ -179,7 +181,14 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
 }
 static cudaError_t copy(const char* what, void* d, const void* s, size_t n, cudaMemcpyKind k) {
     if (note("%s %d %zu %p %p", what, (int)k, n, d, s)) return cudaErrorUnknown;
-    memmove(d, s, n);
+    if (k == cudaMemcpyDeviceToHost) {  // an error where the host may not write, as from the kernel's own copies
+        const int fd = memfd_create("copy", 0);
+        const bool ok = fd >= 0 && pwrite(fd, s, n, 0) == (ssize_t)n && pread(fd, d, n, 0) == (ssize_t)n;
+        close(fd);
+        if (!ok) return cudaErrorInvalidValue;
+    } else {
+        memmove(d, s, n);
+    }
     if (n == sizeof(int) && k == cudaMemcpyDeviceToHost && g_int) memcpy(d, &g_int, n);
     return cudaSuccess;
 }

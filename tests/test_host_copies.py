@@ -1,11 +1,13 @@
 """Which route a host array takes: a kernel that loads and stores its doubles
 in place, or the runtime's copies.  On the stand-in runtime, without a GPU."""
 import ctypes as C
+import mmap
 
 import numpy as np
 import pytest
 
 import _fake_cuda
+from pyflct_gb300 import _lib
 from pyflct_gb300.flct import make_params
 
 
@@ -103,3 +105,48 @@ def test_small_copies_in_are_the_runtimes(host, n, kernel):
     copies = [x.split() for x in log if x.startswith("copy 1 ") and x.split()[2] == str(8 * n * n)]
     assert len(copies) == (0 if kernel else 2)
     assert [int(x.split()[3]) for x in log if "k_copy_arrays" in x] == ([2, 3] if kernel else [3])
+
+
+READ_ONLY = """
+import mmap, sys, ctypes as C, numpy as np
+sys.path[:0] = %r
+import _fake_cuda
+from pyflct_gb300 import _lib
+from pyflct_gb300.flct import make_params
+lib = _lib.load(%r)
+lib.fake_log.restype = C.c_char_p
+lib.fake_reset.argtypes = [C.c_long]
+host, (name, n, nin, nout, k) = _fake_cuda.Host(lib), %r
+out = [np.zeros((n, n)) for _ in range(nout)]
+out[k] = np.frombuffer(mmap.mmap(-1, 8 * n * n, prot=mmap.PROT_READ), np.float64).reshape(n, n)
+p = [C.cast(a.ctypes.data, C.POINTER(C.c_double)) for a in [np.zeros((n, n)) for _ in range(nin)] + out]
+if name == "velocity":
+    rc, log = host.call("velocity", C.byref(make_params(1.0, 1.0, 3.0)), p[0], p[1], n, n, *p[2:])
+elif name == "shift":
+    rc, log = host.call("shift_frac2d", p[0], C.c_double(0.5), C.c_double(0.25), p[1], n, n, 1)
+else:
+    rc, log = host.call("warp_frac2d", *p, n, n, 1)
+assert rc == _lib.ERR_CUDA, rc
+assert sum("k_copy_arrays" in x for x in log) == (1 if 8 * n * n * nin > 32768 else 0)  # the inputs'
+assert log[-1] == "sync stream"
+"""
+
+
+@pytest.mark.parametrize("name", CALLS)
+@pytest.mark.parametrize("n", [N, 12])
+def test_results_the_host_may_not_write_are_not_the_kernels(host, name, n):
+    """A store of the kernel to a page without permission would be the device's fault.  The call
+    ends with an error, or with the host's own fault where the results are less than a page."""
+    import os
+    import signal
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    nin, nout = CALLS[name]
+    for k in range(nout):
+        code = READ_ONLY % ([os.path.dirname(here), here], host.lib._name, (name, n, nin, nout, k))
+        r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
+        if 8 * n * n < mmap.PAGESIZE:
+            assert r.returncode == -signal.SIGSEGV
+        else:
+            assert r.returncode == 0, r.stderr
