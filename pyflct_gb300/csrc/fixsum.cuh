@@ -14,8 +14,10 @@
 // largest); boxes above 64 x 64 take a unit two bits higher, so that their up
 // to 2^14 values stay below 2^127 too.  Spans and runs are fixed by the frame
 // geometry alone, and integer sums are exact, so every box sum is the same
-// for any order, run length or band split, and is rounded once when it
-// becomes a double.
+// for any order of its values and any band split, and is rounded once when it
+// becomes a double.  A long run may take a larger unit than a short one would
+// (at most 2^8 times: box_cols in prepass.cu), and then drops low bits of
+// values 2^54 times smaller than the box's largest.
 // Non-finite inputs are counted instead (NaN, +inf and -inf in 16-bit
 // fields) and give the value a sequential double sum would have: NaN with
 // any NaN or with both infinities, else the infinity present.
