@@ -2317,9 +2317,11 @@ flct_status flct_gpu_velocity(flct_ctx* ctx, const flct_params* p, const double*
     // is settled (a first FLCT_FORM_AUTO call tunes in one band).  Page-locked
     // buffers only, where the bands are a replayed graph: the ~100 stream
     // operations of an eager banded call cost more than their overlap gives
-    // (pageable, five bands against one: 201 x 101 362 against 147 us, 1024^2
-    // -s 4i 870 against 537, 1024^2 every pixel 3,727 against 3,004), unless
-    // FLCT_HOST_BANDS asks for them
+    // (pageable, five bands against one: 201 x 101 335 against 98 us, 1024^2
+    // -s 4i 0.84 against 0.48 ms, every pixel 3.62 against 2.89, 4096^2 -s 4i
+    // 7.6 against 6.8, 8192^2 -s 4i 22.0 against 21.6; with two bands no size
+    // wins either, and results on fresh pages cost several times as much),
+    // unless FLCT_HOST_BANDS asks for them
     const bool locked = page_locked(f1) && page_locked(f2) && page_locked(vx) && page_locked(vy) && page_locked(vm);
     if (locked || ctx->host_bands_asked) {
         Job j;

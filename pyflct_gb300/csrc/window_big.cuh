@@ -151,7 +151,10 @@ __global__ void __launch_bounds__(BigShape<M>::THREADS, BigShape<M>::MINB) k_win
     __syncthreads();
 
     // lane groups of the column passes (eight neighbouring columns, so that
-    // loads from the frames are whole 128-byte lines) and of the row passes
+    // loads from the frames are whole 128-byte lines) and of the row passes.
+    // Groups past the last line take part in the exchanges with the last
+    // line's values (a line of their own warp, read before its owners store)
+    // and store nothing.
     const int cr = ((lane >> 3) & 1) * 2 + (lane >> 4), cl = warp * 8 + (lane & 7);
     const int rr = lane & 3, rl = warp * 8 + (lane >> 2);
 
