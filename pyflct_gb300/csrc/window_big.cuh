@@ -227,11 +227,12 @@ __global__ void __launch_bounds__(BigShape<M>::THREADS, BigShape<M>::MINB) k_win
             __syncthreads();
             // maxima within 2^+-40 of 1 need no scaling: every value of the
             // transforms then stays inside FP32's normal range; else the
-            // columns are done again, each sub-image times an exact power of two
+            // columns are done again, each sub-image times an exact power of
+            // two, or both times zero where one is zero (the correlation is)
             const unsigned b1 = red[0], b2 = red[1];
-            auto near1 = [](unsigned b) { return b == 0u || (b >> 23) - 87u <= 80u; };
+            auto near1 = [](unsigned b) { return (b >> 23) - 87u <= 80u; };
             if (scaled || (near1(b1) && near1(b2))) break;
-            cs = make_float2(pow2_scale(b1), pow2_scale(b2));
+            cs = b1 == 0u || b2 == 0u ? make_float2(0.f, 0.f) : make_float2(pow2_scale(b1), pow2_scale(b2));
             __syncthreads();  // every thread has read the maxima and its part of z
         }
         if (t < 4) s_red[4 * (par ^ 1) + t] = t == 3 ? 0xffffffffu : 0u;  // the next window's

@@ -280,10 +280,13 @@ k_window_fp32(WinArgs a) {
                 b2 = s_max[2 * team + 1];
             }
             // maxima within 2^+-40 of 1 need no scaling: every value of the
-            // transforms then stays inside FP32's normal range
-            auto near1 = [](unsigned b) { return b == 0u || (b >> 23) - 87u <= 80u; };
+            // transforms then stays inside FP32's normal range.  Where one
+            // sub-image is zero the other goes too: the correlation is zero,
+            // not what the other's rounding leaves of the separation
+            auto near1 = [](unsigned b) { return (b >> 23) - 87u <= 80u; };
             if (!(near1(b1) && near1(b2))) {
-                const float2 cs = make_float2(pow2_scale(b1), pow2_scale(b2));
+                const bool flat = b1 == 0u || b2 == 0u;
+                const float2 cs = flat ? make_float2(0.f, 0.f) : make_float2(pow2_scale(b1), pow2_scale(b2));
 #pragma unroll
                 for (int ii = 0; ii < N; ++ii) x[ii] = emul(x[ii], cs);
             }
