@@ -103,6 +103,15 @@ __global__ void k_gz(const double* __restrict__ f1, const double* __restrict__ f
 // 0.113 -> 0.127).
 constexpr int kDftChunk = 16;
 
+// Both frames' exact scales from their maxima.  Where one frame is zero both
+// are: the correlation is zero, not what the other frame's rounding leaves of
+// the separation.
+__device__ __forceinline__ float2 frame_scales(const unsigned* scale) {
+    if (!scale) return make_float2(1.f, 1.f);
+    if (scale[0] == 0u || scale[1] == 0u) return make_float2(0.f, 0.f);
+    return make_float2(pow2_scale(scale[0]), pow2_scale(scale[1]));
+}
+
 template <int DIR, int TL, int LP, int KQ, bool REAL_OUT>
 __global__ void __launch_bounds__(256) k_dft_rows(const float2* __restrict__ in, float2* __restrict__ out, int L,
                                                   int lines, const float2* __restrict__ tw,
@@ -115,7 +124,7 @@ __global__ void __launch_bounds__(256) k_dft_rows(const float2* __restrict__ in,
     // reads whole rows of ws
     const int t = threadIdx.x, tk = t % TK, tl = 2 * (t / TK);
     const int k0 = blockIdx.x * WK, l0 = blockIdx.y * WL;
-    const float c1 = scale ? pow2_scale(scale[0]) : 1.f, c2 = scale ? pow2_scale(scale[1]) : 1.f;
+    const float2 c = frame_scales(scale);
     // this thread's twiddle column, from its row on
     constexpr int WR = 256 / WK;  // twiddle rows a round
     const int wk = t % WK, wj = t / WK, k = min(k0 + wk, L - 1);
@@ -146,8 +155,8 @@ __global__ void __launch_bounds__(256) k_dft_rows(const float2* __restrict__ in,
 #pragma unroll
         for (int q = 0; q < NX; ++q) {
             if (WL * J < 256 && lx >= WL) break;
-            xr[jx][lx + q * (256 / J)] = nx[q].x * c1;
-            xi[jx][lx + q * (256 / J)] = nx[q].y * c2;
+            xr[jx][lx + q * (256 / J)] = nx[q].x * c.x;
+            xi[jx][lx + q * (256 / J)] = nx[q].y * c.y;
         }
 #pragma unroll
         for (int q = 0; q < NW; ++q) {
@@ -202,7 +211,7 @@ __global__ void __launch_bounds__(256) k_dft_long(const float2* __restrict__ in,
     grid_dep_wait();
     const int k = blockIdx.x * 256 + threadIdx.x;
     const float2* const src = in + (size_t)blockIdx.y * L;
-    const float c1 = scale ? pow2_scale(scale[0]) : 1.f, c2 = scale ? pow2_scale(scale[1]) : 1.f;
+    const float2 c = frame_scales(scale);
     float ax = 0.f, ay = 0.f;
     int idx = 0;  // (j k) mod L
     for (int j0 = 0; j0 < L; j0 += J) {
@@ -210,7 +219,7 @@ __global__ void __launch_bounds__(256) k_dft_long(const float2* __restrict__ in,
         __syncthreads();
         for (int j = threadIdx.x; j < jn; j += 256) {
             const float2 v = src[j0 + j];
-            x[j] = make_float2(v.x * c1, v.y * c2);
+            x[j] = make_float2(v.x * c.x, v.y * c.y);
         }
         __syncthreads();
         if (k >= L) continue;

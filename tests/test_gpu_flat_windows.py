@@ -1,4 +1,4 @@
-"""Windows with one flat sub-image: its transform is zero, so is the
+"""Windows and whole frames with one flat image: its transform is zero, so is the
 correlation, and the shift is exactly 0 (as the oracle's), whatever the other
 sub-image holds; its neighbours keep the results they have without it."""
 import numpy as np
@@ -57,3 +57,18 @@ def test_fields_over_a_hole_of_one_frame(sigma, hires):
     assert vx[inside].size and (ox[inside] == (-1 if hires else 0)).all()
     for a, b in ((vx, ox), (vy, oy), (vm, om)):
         assert np.array_equal(a[inside], b[inside])
+
+
+@pytest.mark.parametrize("shape", [(16, 16), (97, 101), (300, 200), (3, 10007)])
+@pytest.mark.parametrize("hires", [False, True])
+@pytest.mark.parametrize("value", [0.0, 1.5])
+def test_whole_frame_flat(shape, hires, value):
+    """sigma = 0 with one frame flat (sums of 1.5 are exact)."""
+    from pyflct_gb300.flct import flct
+    f = np.random.default_rng(shape[1]).standard_normal(shape)
+    for f1, f2 in ((np.full(shape, value), f), (f, np.full(shape, value)), (f * 0 + value, f * 0 - value)):
+        got = [float(np.squeeze(a)) for a in flct(f1, f2, 1.0, 1.0, 0.0, hires=hires)]
+        want = [-1.0, -1.0, 1.0] if hires else [0.0, 0.0, 1.0]
+        assert got == want
+        if max(shape) < 1000:  # (the oracle takes seconds a long line)
+            assert want == [float(np.squeeze(a)) for a in po.velocity(f1, f2, sigma=0.0, hires=hires)]
