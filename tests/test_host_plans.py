@@ -35,7 +35,7 @@ def quickest(host, name, nx, ny):
 @pytest.mark.parametrize("name", ["shift_frac2d", "warp_frac2d"])
 def test_rough_lengths_cost_the_host_no_more(host, name, n):
     smooth = quickest(host, name, 3, 5120)  # a longer line without a convolution
-    assert quickest(host, name, 3, n) <= smooth + 60e-6
+    assert quickest(host, name, 3, n) <= smooth + 100e-6
 
 
 @pytest.mark.parametrize("shape, lines", [((3, 37), False), ((17, 17), False), ((2, 17), False), ((37, 37), False),
